@@ -104,6 +104,17 @@ __device__ __forceinline__ int cell_of(float2 p, const StepParams &s) {
 	return y * s.gx + x;
 }
 
+// r = sqrt(r2) and 1 / r, or r = 0 and 1 for coinciding points (Vec2Normalize
+// keeps a zero vector).  Every particle meets itself in its own list, and the
+// root of 0 would send its warp down the slow path of sqrtf each time; the
+// root of 1 gives the same two results.
+__device__ __forceinline__ float root_and_inverse(float r2, float &r) {
+	const bool zero = r2 == 0.0f;
+	const float len = sqrtf(zero ? 1.0f : r2);
+	r = zero ? 0.0f : len;
+	return 1.0f / len;
+}
+
 __device__ __forceinline__ int rect_dist(int ax0, int ay0, int ax1, int ay1, int bx0, int by0, int bx1, int by1) {
 	int dx = max(0, max(ax0 - bx1, bx0 - ax1));
 	int dy = max(0, max(ay0 - by1, by0 - ay1));
@@ -176,8 +187,9 @@ __global__ void k_integrate(Totals tt, Particles P, SimTables T) {
 template <class C>
 struct ViscSmemT {
 	float2 pos[kStageCap];
-	float2 vel[kStageCap + 2];  // + a scratch slot (kStageCap) for the chains' idle steps
-	float4 geo[3][C::kGeom];  // in-range pairs of a particle, list order: slot, unit vector, 1 - q
+	float2 vel[kStageCap];
+	float4 geo[3][C::kGeom];  // in-range pairs of a particle, list order: byte offset into vel, unit vector, 1 - q
+	float4 idle;              // the entry of a chain without pairs: a valid slot, no direction
 	int m[3];
 	int2 split[3];            // first pair of the middle, first pair of the tail
 	int warpCnt[2][C::kWarps];
@@ -242,7 +254,7 @@ __device__ __forceinline__ void visc_geometry(ViscSmemT<C> &S, int buf, int slot
 			parity ^= 1;
 		}
 		const int at = before + __popc(mask & lanemask_lt());
-		if (in && at < C::kGeom) S.geo[buf][at] = make_float4(__int_as_float(e), rx, ry, r2);
+		if (in && at < C::kGeom) S.geo[buf][at] = make_float4(__int_as_float(8 * e), rx, ry, r2);
 		m += total;
 	}
 	nHead = __reduce_add_sync(kFull, nHead);
@@ -264,140 +276,93 @@ __device__ __forceinline__ void visc_geometry(ViscSmemT<C> &S, int buf, int slot
 	const int mm = min(m, C::kGeom);
 	for (int q = p; q < mm; q += C::kProducers) {
 		const float4 g = S.geo[buf][q];
-		const float r = sqrtf(g.w);
+		float r;  // Vec2Length(Rij) == rij
+		const float inv = root_and_inverse(g.w, r);
 		const float qq = r * s.invH;
-		float len = r;  // Vec2Length(Rij) == rij
-		if (len == 0.0f) len = 1.0f;
-		const float inv = 1.0f / len;
 		S.geo[buf][q] = make_float4(g.x, g.y * inv, g.z * inv, 1.0f - qq);
 	}
 	if (p == 0) S.m[buf] = m;
 }
 
-// The serial part of the viscosity pass for one particle, in list order
-// (sph.h:497-512, demo4.cpp:231-234): v_i carries from pair to pair.  Each
-// slot occurs once per list, so the next pairs' velocities may be loaded
-// before this pair's store.  The impulse (f n * 0.5) * dt is computed as
+// One pair of a particle's viscosity chain (sph.h:497-512, demo4.cpp:231-234):
+// v_i carries from pair to pair.  The impulse (f n * 0.5) * dt is computed as
 // (f n) * (0.5 dt): 0.5 dt is exact and halving is exact, so both round the
-// same real product once (unless |f n| < 2^-125).
-template <bool kBranchy>
-__device__ __forceinline__ void visc_pair(float2 *vel, int j, float2 n, float o, float2 vj, float2 &vi, float sigma,
-                                          float beta, float hdt) {
-	// Only approaching pairs (u > 0) exchange an impulse: computed
-	// unconditionally and selected, or (kBranchy) skipped.
+// same real product once (unless |f n| < 2^-125).  Only approaching pairs
+// (u > 0) exchange an impulse; `live` masks the idle steps of a shorter chain.
+// The impulse is computed unconditionally and applied by predicated
+// instructions, so a pair's dependent chain is ten FP32 operations and
+// neither a select nor a branch ends it (a branch costs nine cycles a pair).
+__device__ __forceinline__ void visc_pair(uint32_t at, float2 n, float o, float2 vj, float2 &vi, float sigma,
+                                          float beta, float hdt, bool live = true) {
 	const float uu = (vi.x - vj.x) * n.x + (vi.y - vj.y) * n.y;
-	if (kBranchy) {
-		if (uu > 0.0f) {
-			const float f = o * (sigma * uu + beta * (uu * uu));
-			const float ix = (f * n.x) * hdt;
-			const float iy = (f * n.y) * hdt;
-			vi.x = vi.x - ix;
-			vi.y = vi.y - iy;
-			vel[j] = make_float2(ix + vj.x, iy + vj.y);
-		}
-		return;
-	}
 	const float f = o * (sigma * uu + beta * (uu * uu));
 	const float ix = (f * n.x) * hdt;
 	const float iy = (f * n.y) * hdt;
-	const bool ap = uu > 0.0f;
-	vi.x = ap ? vi.x - ix : vi.x;
-	vi.y = ap ? vi.y - iy : vi.y;
-	vel[j] = ap ? make_float2(ix + vj.x, iy + vj.y) : vj;
+	const float wx = ix + vj.x, wy = iy + vj.y;
+	asm volatile(
+	    "{\n"
+	    ".reg .pred q, p;\n"
+	    "setp.ne.s32 q, %8, 0;\n"
+	    "setp.gt.and.f32 p, %2, 0f00000000, q;\n"
+	    "@p sub.rn.f32 %0, %0, %3;\n"
+	    "@p sub.rn.f32 %1, %1, %4;\n"
+	    "@p st.shared.v2.f32 [%5], {%6, %7};\n"
+	    "}\n"
+	    : "+f"(vi.x), "+f"(vi.y)
+	    : "f"(uu), "f"(ix), "f"(iy), "r"(at), "f"(wx), "f"(wy), "r"((int)live)
+	    : "memory");
 }
 
-// The chain over m buffered pairs G (slot, unit vector, 1 - q) with the
-// velocities vel.  Software pipeline: the geometry and partner velocities of
-// the next kU pairs are loaded while the chain runs over the current kU.
-template <bool kBranchy, int kU>
-__device__ __forceinline__ void visc_run(float2 *vel, const float4 *G, int m, float2 &vi, float sigma, float beta,
-                                         float hdt) {
-	float4 g[kU];
-	float2 vj[kU];
-#pragma unroll
-	for (int u = 0; u < kU; ++u) g[u] = u < m ? G[u] : make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-	for (int u = 0; u < kU; ++u) vj[u] = vel[__float_as_int(g[u].x)];
-	int q = 0;
-	for (; q + 2 * kU <= m; q += kU) {
-		float4 gn[kU];
-		float2 vn[kU];
-#pragma unroll
-		for (int u = 0; u < kU; ++u) gn[u] = G[q + kU + u];
-#pragma unroll
-		for (int u = 0; u < kU; ++u) vn[u] = vel[__float_as_int(gn[u].x)];
-#pragma unroll
-		for (int u = 0; u < kU; ++u)
-			visc_pair<kBranchy>(vel, __float_as_int(g[u].x), make_float2(g[u].y, g[u].z), g[u].w, vj[u], vi, sigma,
-			                    beta, hdt);
-#pragma unroll
-		for (int u = 0; u < kU; ++u) {
-			g[u] = gn[u];
-			vj[u] = vn[u];
-		}
-	}
-	// At most 2 kU - 1 pairs left, the first kU of them loaded.
-	if (q + kU <= m) {
-		float4 gn[kU];
-		float2 vn[kU];
-#pragma unroll
-		for (int u = 0; u < kU; ++u) gn[u] = q + kU + u < m ? G[q + kU + u] : make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-		for (int u = 0; u < kU; ++u) vn[u] = vel[__float_as_int(gn[u].x)];
-#pragma unroll
-		for (int u = 0; u < kU; ++u)
-			visc_pair<kBranchy>(vel, __float_as_int(g[u].x), make_float2(g[u].y, g[u].z), g[u].w, vj[u], vi, sigma,
-			                    beta, hdt);
-#pragma unroll
-		for (int u = 0; u < kU; ++u) {
-			g[u] = gn[u];
-			vj[u] = vn[u];
-		}
-		q += kU;
-	}
-#pragma unroll
-	for (int u = 0; u < kU; ++u)
-		if (q + u < m)
-			visc_pair<kBranchy>(vel, __float_as_int(g[u].x), make_float2(g[u].y, g[u].z), g[u].w, vj[u], vi, sigma,
-			                    beta, hdt);
+__device__ __forceinline__ uint32_t shared_addr(const void *p) {
+	return (uint32_t)__cvta_generic_to_shared(p);
+}
+__device__ __forceinline__ float2 vel_at(const float2 *vel, int off) {
+	return *reinterpret_cast<const float2 *>(reinterpret_cast<const char *>(vel) + off);
 }
 
-// The chain over pairs [start, start + len) of G, in lockstep with the
-// other chain lane: both run n >= len steps (the longer of the two).  This
-// lane's steps past len take an idle pair: the scratch slot kStageCap with a
-// zero unit vector, so u = 0 is not approaching and neither velocity
-// changes; the steps stay branch-free.  Software pipeline: the next kU pairs'
-// geometry and partner velocities load while the chain runs the current kU
-// (two measured fastest: 1.32 ms for the 65,536-particle sweep against 1.51
-// with four and 1.42 with eight).  The two lanes touch disjoint slots, so a
-// prefetched velocity is never one the other lane changes.
-template <bool kBranchy>
-__device__ __forceinline__ void visc_run_range(float2 *vel, const float4 *G, int start, int len, int n, float2 &vi,
-                                               float sigma, float beta, float hdt) {
-	constexpr int kU = 2;
-	const float4 idle = make_float4(__int_as_float(kStageCap), 0.f, 0.f, 0.f);
-	float4 g[kU];
-	float2 vj[kU];
+// The ordered chain over the len buffered pairs G[0..len) (byte offset of the
+// partner's velocity, unit vector, 1 - q), in lockstep with the warp's other
+// chains: all run the n >= len steps of the longest.  Steps past len are
+// masked; they reload entry len - 1 (`idle`, an entry naming a valid slot,
+// when there is none), so no step reads past the buffer.  Software pipeline
+// in groups of four pairs: a group's partner velocities load while the group
+// before it runs, its geometry one group earlier still, so neither
+// shared-memory latency is on the chain.  Each slot occurs once per list and
+// the chains touch disjoint slots, so a prefetched velocity is never one that
+// changes meanwhile.  The loop leaves after whole pairs of groups: a branch
+// costs more than the masked steps it would save.  In isolation, cycles per
+// pair of 112: 53, against 68 for loads two pairs ahead and 61 for one pair's
+// loads between every two pairs; ten dependent operations alone take 47.
+__device__ __forceinline__ void visc_chain(const float2 *vel, const float4 *G, const float4 *idle, int len, int n,
+                                           float2 &vi, float sigma, float beta, float hdt) {
+	const float4 *src = len > 0 ? G : idle;
+	const int last = max(len - 1, 0);
+	const uint32_t base = shared_addr(vel);
+	float4 g[4], h[4];
+	float2 v[4], w[4];
 #pragma unroll
-	for (int u = 0; u < kU; ++u) g[u] = u < len ? G[start + u] : idle;
+	for (int u = 0; u < 4; ++u) g[u] = src[min(u, last)];
 #pragma unroll
-	for (int u = 0; u < kU; ++u) vj[u] = vel[__float_as_int(g[u].x)];
-	for (int q = 0; q < n; q += kU) {
-		float4 gn[kU];
-		float2 vn[kU];
+	for (int u = 0; u < 4; ++u) v[u] = vel_at(vel, __float_as_int(g[u].x));
 #pragma unroll
-		for (int u = 0; u < kU; ++u) gn[u] = q + kU + u < len ? G[start + q + kU + u] : idle;
+	for (int u = 0; u < 4; ++u) h[u] = src[min(4 + u, last)];
+	for (int q = 0; q < n; q += 8) {
 #pragma unroll
-		for (int u = 0; u < kU; ++u) vn[u] = vel[__float_as_int(gn[u].x)];
+		for (int u = 0; u < 4; ++u) w[u] = vel_at(vel, __float_as_int(h[u].x));
 #pragma unroll
-		for (int u = 0; u < kU; ++u)
-			visc_pair<kBranchy>(vel, __float_as_int(g[u].x), make_float2(g[u].y, g[u].z), g[u].w, vj[u], vi, sigma,
-			                    beta, hdt);
+		for (int u = 0; u < 4; ++u)
+			visc_pair(base + __float_as_uint(g[u].x), make_float2(g[u].y, g[u].z), g[u].w, v[u], vi, sigma, beta, hdt,
+			          q + u < len);
 #pragma unroll
-		for (int u = 0; u < kU; ++u) {
-			g[u] = gn[u];
-			vj[u] = vn[u];
-		}
+		for (int u = 0; u < 4; ++u) g[u] = src[min(q + 8 + u, last)];
+#pragma unroll
+		for (int u = 0; u < 4; ++u)
+			visc_pair(base + __float_as_uint(h[u].x), make_float2(h[u].y, h[u].z), h[u].w, w[u], vi, sigma, beta, hdt,
+			          q + 4 + u < len);
+#pragma unroll
+		for (int u = 0; u < 4; ++u) v[u] = vel_at(vel, __float_as_int(g[u].x));
+#pragma unroll
+		for (int u = 0; u < 4; ++u) h[u] = src[min(q + 12 + u, last)];
 	}
 }
 
@@ -430,11 +395,18 @@ __device__ __forceinline__ void visc_wave(ViscSmemT<C> &S, int k, int cnt, int o
 			len = inl ? 0 : m - sp.y;
 		}
 	}
+	const float4 *G = S.geo[buf];
+	// The middle's pairs (at most three): geometry now, velocities later.
+	const int mid = has && head && m <= C::kGeom ? sp.y - sp.x : 0;
+	float4 gm[3];
+#pragma unroll
+	for (int u = 0; u < 3; ++u) gm[u] = u < mid ? G[sp.x + u] : S.idle;
 	const int n = max(len, __shfl_xor_sync(0x3u, len, 1));
-	visc_run_range<C::kBranchy>(S.vel, S.geo[buf], start, len, n, vi, s.sigma, s.beta, hdt);
+	visc_chain(S.vel, G + start, &S.idle, len, n, vi, s.sigma, s.beta, hdt);
 	if (has && !head) S.vel[own + k - 1] = vi;  // particle k - 1 is finished
 	__syncwarp(0x3u);
 	if (!(has && head)) return;
+	const uint32_t base = shared_addr(S.vel);
 	if (m > C::kGeom) {
 		const float2 xi = S.pos[own + k];
 		for (int e = 0; e < L; ++e) {
@@ -447,17 +419,17 @@ __device__ __forceinline__ void visc_wave(ViscSmemT<C> &S, int k, int cnt, int o
 			float lenr = r;
 			if (lenr == 0.0f) lenr = 1.0f;
 			const float inv = 1.0f / lenr;
-			visc_pair<C::kBranchy>(S.vel, e, make_float2(rx * inv, ry * inv), 1.0f - qq, S.vel[e], vi, s.sigma,
-			                       s.beta, hdt);
+			visc_pair(base + 8u * e, make_float2(rx * inv, ry * inv), 1.0f - qq, S.vel[e], vi, s.sigma, s.beta, hdt);
 		}
 		return;
 	}
-	const float4 *G = S.geo[buf];
-	for (int q = sp.x; q < sp.y; ++q) {
-		const float4 g = G[q];
-		const int j = __float_as_int(g.x);
-		visc_pair<C::kBranchy>(S.vel, j, make_float2(g.y, g.z), g.w, S.vel[j], vi, s.sigma, s.beta, hdt);
-	}
+	float2 vm[3];
+#pragma unroll
+	for (int u = 0; u < 3; ++u) vm[u] = vel_at(S.vel, __float_as_int(gm[u].x));
+#pragma unroll
+	for (int u = 0; u < 3; ++u)
+		visc_pair(base + __float_as_uint(gm[u].x), make_float2(gm[u].y, gm[u].z), gm[u].w, vm[u], vi, s.sigma, s.beta,
+		          hdt, u < mid);
 }
 
 }  // namespace
@@ -469,6 +441,7 @@ __global__ void __launch_bounds__(C::kWarps * kWarp, C::kMinBlocks) k_viscosity(
 	ViscSmemT<C> &S = *reinterpret_cast<ViscSmemT<C> *>(smem_raw);
 	const int tid = threadIdx.x, warp = tid / kWarp;
 	const int nLive = *T.nLive;
+	if (tid == 0) S.idle = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
 	for (;;) {
 		if (tid == 0) S.task = atomicAdd(&T.taskCounter[0], 1);
 		__syncthreads();
@@ -577,12 +550,13 @@ __global__ void __launch_bounds__(C::kWarps * kWarp, C::kMinBlocks) k_viscosity(
 template <class C>
 struct ViscSlotT {
 	float2 vel[kStageCap];    // velocities of the 3x3 block, list order
-	float4 geo[2][C::kGeom];  // per buffer: in-range pairs (slot, unit vector, 1 - q) of one particle
+	float4 geo[2][C::kGeom];  // per buffer: in-range pairs (byte offset into vel, unit vector, 1 - q) of one particle
 	float4 pad;               // consecutive slots start 16 bytes apart in the bank space
 };
 template <class C>
 struct ViscMultiSmemT {
 	ViscSlotT<C> slot[C::kSlots];
+	float4 idle;  // the entry of a chain without pairs
 	int segStart[C::kSlots][9], segOff[C::kSlots][9];
 	int state[C::kSlots], task[C::kSlots], first[C::kSlots], cnt[C::kSlots], own[C::kSlots], L[C::kSlots],
 	    k[C::kSlots], cell[C::kSlots], claim[C::kSlots];
@@ -629,7 +603,7 @@ __device__ __forceinline__ void slot_geometry(ViscMultiSmemT<C> &S, int s, int k
 			const bool in = e < L && r2 < h2;
 			const unsigned mask = __ballot_sync(kFull, in);
 			const int at = m + __popc(mask & lanemask_lt());
-			if (in && at < C::kGeom) G[at] = make_float4(__int_as_float(e), rx, ry, r2);
+			if (in && at < C::kGeom) G[at] = make_float4(__int_as_float(8 * e), rx, ry, r2);
 			m += __popc(mask);
 		}
 	}
@@ -637,11 +611,9 @@ __device__ __forceinline__ void slot_geometry(ViscMultiSmemT<C> &S, int s, int k
 	const int mm = min(m, C::kGeom);
 	for (int q = lane; q < mm; q += kWarp) {
 		const float4 g = G[q];
-		const float r = sqrtf(g.w);
+		float r;  // Vec2Length(Rij) == rij
+		const float inv = root_and_inverse(g.w, r);
 		const float qq = r * invH;
-		float len = r;  // Vec2Length(Rij) == rij
-		if (len == 0.0f) len = 1.0f;
-		const float inv = 1.0f / len;
 		G[q] = make_float4(g.x, g.y * inv, g.z * inv, 1.0f - qq);
 	}
 	if (lane == 0) S.m[s][buf] = m;
@@ -811,13 +783,15 @@ __device__ __forceinline__ void slot_produce(ViscMultiSmemT<C> &S, int s, const 
 	}
 }
 
-// The chain of slot s's current particle (lane s of warp 0).
+// The chain of slot s's current particle (lane s of warp 0; `running` is the
+// mask of the lanes that run one).
 template <class C>
-__device__ __forceinline__ void slot_chain(ViscMultiSmemT<C> &S, int s, const Particles &P) {
+__device__ __forceinline__ void slot_chain(ViscMultiSmemT<C> &S, int s, unsigned running, const Particles &P) {
 	const int k = S.k[s], buf = k & 1, m = S.m[s][buf];
 	const int own = S.own[s] + k;
 	float2 *V = S.slot[s].vel;
 	const float sigma = S.sigma[s], beta = S.beta[s], hdt = S.hdt[s];
+	const uint32_t base = shared_addr(V);
 	float2 vi = V[own];
 	if (m > C::kGeom) {
 		// More in-range pairs than the geometry buffer holds: the same pair
@@ -841,11 +815,11 @@ __device__ __forceinline__ void slot_chain(ViscMultiSmemT<C> &S, int s, const Pa
 			float len = r;
 			if (len == 0.0f) len = 1.0f;
 			const float inv = 1.0f / len;
-			visc_pair<false>(V, e, make_float2(rx * inv, ry * inv), 1.0f - qq, V[e], vi, sigma, beta, hdt);
+			visc_pair(base + 8u * e, make_float2(rx * inv, ry * inv), 1.0f - qq, V[e], vi, sigma, beta, hdt);
 		}
-	} else {
-		visc_run<false, 4>(V, S.slot[s].geo[buf], m, vi, sigma, beta, hdt);
 	}
+	const int len = m > C::kGeom ? 0 : m;
+	visc_chain(V, S.slot[s].geo[buf], &S.idle, len, __reduce_max_sync(running, len), vi, sigma, beta, hdt);
 	V[own] = vi;
 }
 
@@ -865,6 +839,7 @@ __global__ void __launch_bounds__(C::kWarps * kWarp, C::kMinBlocks) k_viscosity_
 	if (tid == 0) {
 		S.exhausted = 0;
 		S.aborted = 0;
+		S.idle = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
 	}
 	__syncthreads();
 	for (;;) {
@@ -886,7 +861,9 @@ __global__ void __launch_bounds__(C::kWarps * kWarp, C::kMinBlocks) k_viscosity_
 		const int anyBusy = __syncthreads_or(busy);
 		if ((!anyBusy && S.exhausted) || S.aborted) break;
 		if (warp == 0) {
-			if (lane < C::kSlots && S.state[lane] == kSlotRun) slot_chain<C>(S, lane, P);
+			const bool run = lane < C::kSlots && S.state[lane] == kSlotRun;
+			const unsigned running = __ballot_sync(kFull, run);
+			if (run) slot_chain<C>(S, lane, running, P);
 		} else {
 			if (tid == kWarp && ld_acquire(T.abort) != 0u) S.aborted = 1;
 			__syncwarp();

@@ -11,7 +11,6 @@ namespace sphgb {
 // tasks per SM for many scenes).  Results do not depend on the shape.
 struct ViscWide {
 	static constexpr int kWarps = 4, kProducers = 3 * kWarp, kGeom = 512, kMinBlocks = 4;
-	static constexpr bool kBranchy = false;
 };
 // Lean viscosity: kSlots tasks per block; warp 0's lanes run their chains,
 // kProd producer warps serve them (k_viscosity_multi).
