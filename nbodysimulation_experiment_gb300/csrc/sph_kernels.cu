@@ -1569,16 +1569,18 @@ __global__ void __launch_bounds__(kDensWarps * kWarp, 4) k_density(Totals tt, Pa
 // warps, one block per SM (short per-particle latency, one scene); mid is
 // pipelined with seven, two blocks per SM; lean is two warps without the
 // pipeline and with smaller staging (more tasks per SM, many scenes).
+constexpr int kSumPad = 32;  // +0 entries past the last half, at most one batch of the sum
 template <class C>
 struct DeltaSmemT {
 	static constexpr int kProd = C::kWarps - 1;         // producer warps
 	static constexpr int kPass = kProd * C::kChainW;    // list entries per pipelined particle
 	static constexpr int kSeqPass = C::kWarps * C::kChainW;  // list entries per pass, whole block
-	static constexpr int kHalf = (kSeqPass > kPass ? kSeqPass : kPass) + 16;
+	static constexpr int kHalf = (kSeqPass > kPass ? kSeqPass : kPass) + 36;  // 4 past a multiple of the 32 banks
 	static constexpr int kPhases = C::kPipelined ? 2 : 1;  // half buffers
 	float2 pos[C::kStage];
 	float4 cand[C::kWarps][C::kChainW];  // per warp: in-range candidates: slot, x_j.x, x_j.y, r2
-	float2 half[kPhases][kHalf];  // per phase: delta * 0.5 of the in-range pairs, list order, +0 padded
+	alignas(16) float half[kPhases][2][kHalf];  // per phase, x and y: delta * 0.5 of the in-range pairs, list order, +0 padded
+	alignas(16) unsigned char wcnt8[16];      // kDirect: per warp, in-range pairs of this phase's particle
 	int4 meta[2];             // per phase: pairs, reserved index of (k, k-1) or -1, own slot
 	float2 ownAfter[2];       // per phase: the particle's position after its self pair
 	int4 pslot[C::kPrefetch];  // prefetched per particle: row ranges' first slots, own slot (or -1)
@@ -1728,43 +1730,42 @@ __device__ __forceinline__ void particle_slots(DeltaSmemT<C> &S, const Region &R
 		own = -1;
 	}
 	slot = make_int4(o[0], o[1], o[2], own);
-	len = make_int4(n[0], n[1], n[2], 0);
+	const int L = n[0] + n[1] + n[2];
+	len = make_int4(n[0], n[1], n[2], (L + DeltaSmemT<C>::kProd - 1) / DeltaSmemT<C>::kProd);
 }
 
 // delta * 0.5 of one in-range pair (sph.h:483-495 with demo4.cpp:250-251):
 // particle at xk with pressures pk, neighbour at xj, r2 = |xj - xk|^2.
 __device__ __forceinline__ float2 delta_half(float2 xj, float2 xk, float r2, float2 pk, const StepParams &s) {
 	const float rx = xj.x - xk.x, ry = xj.y - xk.y;
-	const float rij = sqrtf(r2);
-	float len = rij;
-	if (len == 0.0f) len = 1.0f;
-	const float inv = 1.0f / len;
+	float rij;
+	const float inv = root_and_inverse(r2, rij);
 	const float nx = rx * inv, ny = ry * inv;
 	const float term = 1.0f - rij * s.invH;
 	const float d = s.dt2 * (pk.x * term + pk.y * (term * term));
 	return make_float2(d * nx * 0.5f, d * ny * 0.5f);
 }
 
-// dx -= delta * 0.5 over the n buffered halves, in list order
-// (demo4.cpp:251), in batches of eight loaded one batch ahead.  The buffer
-// is padded with +0 for sixteen entries past n, and dx - (+0) == dx exactly.
-__device__ __forceinline__ void sum_halves(const float2 *H, int n, float2 &dx) {
-	float2 h[8];
+// dx -= delta * 0.5 over the n buffered halves of one component, in list
+// order (demo4.cpp:251), starting at dx: one dependent subtraction per pair
+// (four cycles), in batches of 32 loaded at once, so that a batch's loads and
+// its loop branch cost little beside them.  The buffer is padded with +0 for
+// kSumPad entries past n, and dx - (+0) == dx exactly.  Two lanes take a
+// component each.  In isolation 112 pairs take 685 cycles, 818 in batches of
+// eight; one lane subtracting both components took 9.4 cycles a pair.
+__device__ __forceinline__ float sum_halves(const float *H, int n, float dx) {
+	const float4 *H4 = reinterpret_cast<const float4 *>(H);
+	for (int b = 0; b < n; b += kSumPad) {
+		float4 a[kSumPad / 4];
 #pragma unroll
-	for (int u = 0; u < 8; ++u) h[u] = H[u];
-	for (int b = 8; b < n + 8; b += 8) {
-		float2 hn[8];
+		for (int u = 0; u < kSumPad / 4; ++u) a[u] = H4[b / 4 + u];
 #pragma unroll
-		for (int u = 0; u < 8; ++u) hn[u] = H[b + u];
-#pragma unroll
-		for (int u = 0; u < 8; ++u) {
-			dx.x = dx.x - h[u].x;
-			dx.y = dx.y - h[u].y;
-		}
-#pragma unroll
-		for (int u = 0; u < 8; ++u) h[u] = hn[u];
+		for (int u = 0; u < kSumPad / 4; ++u) dx = dx - a[u].x - a[u].y - a[u].z - a[u].w;
 	}
+	return dx;
 }
+__device__ __forceinline__ float comp(float2 v, int c) { return c == 0 ? v.x : v.y; }
+__device__ __forceinline__ float *comp_of(float2 *v, int c) { return reinterpret_cast<float *>(v) + c; }
 
 // Scan and compaction of one particle's list entries [p0, p0 + pl) over
 // `nw` warps (this thread is warp `w` of them): each warp takes a contiguous
@@ -1814,8 +1815,7 @@ __device__ __forceinline__ void relax_particle(DeltaSmemT<C> &S, int4 sl, int4 l
 	if (own < 0) return;  // index check failed (uniform)
 	const int len0 = ln.x, l01 = ln.x + ln.y, L = l01 + ln.z;
 	const float2 xk = S.pos[own];
-	float2 *H = S.half[0];
-	float2 dx = make_float2(0.0f, 0.0f);  // thread 0
+	float dx = 0.0f;  // threads 0 and 1: x and y
 	for (int p0 = 0; p0 < L; p0 += kPass) {
 		const int pl = min(L - p0, kPass);
 		const int cnt = scan_range(S.cand[warp], kW, warp, lane, p0, pl, sl, len0, l01, xk, own, -1, S.pos, s.h2,
@@ -1829,7 +1829,7 @@ __device__ __forceinline__ void relax_particle(DeltaSmemT<C> &S, int4 sl, int4 l
 			before += (w < warp) ? c : 0;
 			total += c;
 		}
-		if (tid < 16) H[total + tid] = make_float2(0.0f, 0.0f);
+		if (tid < kSumPad) S.half[0][0][total + tid] = S.half[0][1][total + tid] = 0.0f;
 		for (int q = lane; q < cnt; q += kWarp) {
 			const float4 cd = S.cand[warp][q];
 			const float2 xj = make_float2(cd.y, cd.z);
@@ -1837,34 +1837,28 @@ __device__ __forceinline__ void relax_particle(DeltaSmemT<C> &S, int4 sl, int4 l
 			const int slot = __float_as_int(cd.x);
 			const float2 moved = make_float2(h.x + xj.x, h.y + xj.y);
 			if (slot == own) S.ownAfter[0] = moved; else S.pos[slot] = moved;
-			H[before + q] = h;
+			S.half[0][0][before + q] = h.x;
+			S.half[0][1][before + q] = h.y;
 		}
 		__syncthreads();
-		if (tid == 0) {
-			sum_halves(H, total, dx);
-			if (p0 + kPass >= L) {
-				const float2 xo = S.ownAfter[0];
-				S.pos[own] = make_float2(dx.x + xo.x, dx.y + xo.y);
-			}
+		if (tid < 2) {
+			dx = sum_halves(S.half[0][tid], total, dx);
+			if (p0 + kPass >= L) *comp_of(&S.pos[own], tid) = dx + comp(S.ownAfter[0], tid);
 		}
 		__syncthreads();
 	}
 }
 
-// Summer warp, lane 0: finish the particle of phase buffer b (fill its
-// reserved pair with hres, its ordered dx sum, its final position).
-// Returns the final position.
+// Summer warp, lanes c = 0 and 1 (x and y): the ordered dx sum of the
+// particle of phase buffer b, its reserved pair filled with hres (this
+// component's D/2).  Returns the component of its final position.
 template <class C>
-__device__ __forceinline__ float2 finish_particle(DeltaSmemT<C> &S, int b, float2 hres) {
+__device__ __forceinline__ float finish_sum(DeltaSmemT<C> &S, int b, int c, float hres) {
 	const int4 m = S.meta[b];
-	float2 *H = S.half[b];
+	float *H = S.half[b][c];
+	const float xo = comp(S.ownAfter[b], c);
 	if (m.y >= 0) H[m.y] = hres;
-	float2 dx = make_float2(0.0f, 0.0f);
-	sum_halves(H, m.x, dx);
-	const float2 xo = S.ownAfter[b];
-	const float2 xp = make_float2(dx.x + xo.x, dx.y + xo.y);
-	S.pos[m.z] = xp;
-	return xp;
+	return sum_halves(H, m.x, 0.0f) + xo;
 }
 
 template <class C>
@@ -1883,7 +1877,6 @@ __device__ __forceinline__ void produce(DeltaSmemT<C> &S, int b, int4 sl, int4 l
 	const int own = sl.w;
 	const int len0 = ln.x, l01 = ln.x + ln.y, L = l01 + ln.z;
 	const float2 xk = S.pos[own];
-	float2 *H = S.half[b];
 	if (tid == 0) S.meta[b].y = -1;
 	const int cnt = scan_range(S.cand[warp], kP, warp, lane, 0, L, sl, len0, l01, xk, own, prev, S.pos, s.h2,
 	                           &S.ownAfter[b]);
@@ -1901,7 +1894,7 @@ __device__ __forceinline__ void produce(DeltaSmemT<C> &S, int b, int4 sl, int4 l
 	} else {
 		__syncwarp();
 	}
-	if (tid < 16) H[total + tid] = make_float2(0.0f, 0.0f);
+	if (tid < kSumPad) S.half[b][0][total + tid] = S.half[b][1][total + tid] = 0.0f;
 	for (int q = lane; q < cnt; q += kWarp) {
 		const float4 cd = S.cand[warp][q];
 		if (cd.w < 0.0f) {
@@ -1913,7 +1906,8 @@ __device__ __forceinline__ void produce(DeltaSmemT<C> &S, int b, int4 sl, int4 l
 		const int slot = __float_as_int(cd.x);
 		const float2 moved = make_float2(h.x + xj.x, h.y + xj.y);
 		if (slot == own) S.ownAfter[b] = moved; else S.pos[slot] = moved;
-		H[before + q] = h;
+		S.half[b][0][before + q] = h.x;
+		S.half[b][1][before + q] = h.y;
 	}
 	if (tid == 0) {
 		S.meta[b].x = total;
@@ -1921,26 +1915,112 @@ __device__ __forceinline__ void produce(DeltaSmemT<C> &S, int b, int4 sl, int4 l
 	}
 }
 
-// Summer's part of phase b (lane 0): finish the previous particle (buffer
-// b ^ 1), then evaluate the pair (k, k-1) of particle k (list slots sl, ln,
-// pressures pk) if k-1 is in k's list; its D/2 goes to hres.
+// Direct form of produce (kDirect): warp w takes a contiguous range of the
+// list, entry `at[i]` (a staged slot, or -1) of this thread in round i of R,
+// and evaluates it without compacting first, so the square root and the
+// division run beside the counting and only the halves' places wait for the
+// other warps' counts.  R is a compile-time number: a uniform branch per round
+// costs as much as the round's arithmetic.  With the two-lane sum below, one
+// task of 36 particles with 324 list entries (wide shape, alone): 1,720 cycles
+// per particle, 2,060 when every warp compacted first.
+template <class C, int R>
+__device__ __forceinline__ void produce_direct(DeltaSmemT<C> &S, int b, const int *at, int own, float2 pk, int prev,
+                                               uint4 below, const StepParams &s, int tid) {
+	constexpr int kP = DeltaSmemT<C>::kProd;
+	static_assert(kP <= 16 && C::kChainW < 256, "a phase's counts are one 16-byte word");
+	const int lane = tid & (kWarp - 1), warp = tid / kWarp;
+	const float2 xk = S.pos[own];
+	float2 xj[R], h[R];
+	unsigned mask[R];
+	bool in[R];
+	int cnt = 0;
+	if (tid == 0) S.meta[b] = make_int4(0, -1, own, 0);
+#pragma unroll
+	for (int i = 0; i < R; ++i) xj[i] = S.pos[max(at[i], 0)];
+#pragma unroll
+	for (int i = 0; i < R; ++i) {
+		const float rx = xj[i].x - xk.x, ry = xj[i].y - xk.y;
+		const float r2 = rx * rx + ry * ry;
+		// (k, k-1) keeps its place whatever its distance: the summer
+		// evaluates it.
+		in[i] = at[i] >= 0 && at[i] != prev && r2 < s.h2;
+		mask[i] = __ballot_sync(kFull, in[i] || (at[i] >= 0 && at[i] == prev));
+		cnt += __popc(mask[i]);
+		h[i] = delta_half(xj[i], xk, r2, pk, s);
+	}
+	if (lane == 0) S.wcnt8[warp] = (unsigned char)cnt;
+#pragma unroll
+	for (int i = 0; i < R; ++i) {
+		const float2 moved = make_float2(h[i].x + xj[i].x, h[i].y + xj[i].y);
+		if (at[i] == own) S.ownAfter[b] = in[i] ? moved : xj[i];
+		else if (in[i]) S.pos[at[i]] = moved;
+	}
+	producers_bar<C>();
+	const uint4 c4 = *reinterpret_cast<const uint4 *>(S.wcnt8);
+	// Sum of the earlier warps' counts: bytes, masked once per task.
+	int before = (int)(__dp4a(c4.x & below.x, 0x01010101u, 0u) + __dp4a(c4.y & below.y, 0x01010101u, 0u) +
+	                   __dp4a(c4.z & below.z, 0x01010101u, 0u) + __dp4a(c4.w & below.w, 0x01010101u, 0u));
+	if (warp == kP - 1) {
+		const int total = before + cnt;
+		S.half[b][0][total + lane] = S.half[b][1][total + lane] = 0.0f;
+		if (lane == 0) S.meta[b].x = total;
+	}
+#pragma unroll
+	for (int i = 0; i < R; ++i) {
+		const int place = before + __popc(mask[i] & lanemask_lt());
+		if (in[i]) {
+			S.half[b][0][place] = h[i].x;
+			S.half[b][1][place] = h[i].y;
+		} else if (at[i] >= 0 && at[i] == prev) {
+			S.meta[b].y = place;
+		}
+		before += __popc(mask[i]);
+	}
+}
+
+// Byte mask of the counts of the warps before this one.
+__device__ __forceinline__ uint4 warps_below(int warp) {
+	uint32_t m[4];
+#pragma unroll
+	for (int q = 0; q < 4; ++q) {
+		const int n = min(max(warp - 4 * q, 0), 4);
+		m[q] = n == 4 ? 0xffffffffu : (1u << (8 * n)) - 1u;
+	}
+	return make_uint4(m[0], m[1], m[2], m[3]);
+}
+
+// The list entry of this producer thread in round i (a staged slot, or -1) for
+// the particle with row ranges sl, ln.
 template <class C>
-__device__ __forceinline__ void summer(DeltaSmemT<C> &S, int b, int4 sl, int4 ln, float2 pk, const StepParams &s,
-                                       float2 &hres) {
-	const int prev = S.meta[b ^ 1].z;
-	const float2 xp = finish_particle<C>(S, b ^ 1, hres);
-	hres = make_float2(0.0f, 0.0f);
+__device__ __forceinline__ int direct_slot(int4 sl, int4 ln, int tid, int i) {
+	const int r = i * kWarp + (tid & (kWarp - 1));
+	const int e = (tid / kWarp) * ln.w + r;
+	const int l01 = ln.x + ln.y;
+	// Rows start at sl.x, sl.y - ln.x and sl.z - l01 of the flat list.
+	const int base = e < ln.x ? sl.x : (e < l01 ? sl.y - ln.x : sl.z - l01);
+	return r < ln.w && e < l01 + ln.z ? base + e : -1;
+}
+
+// Summer's part of a phase (lanes c = 0 and 1 of the warp: x and y): finish
+// the previous particle `prev` (buffer b ^ 1), then evaluate the pair (k, k-1)
+// of particle k (list slots sl, ln, pressures pk) if k-1 is in k's list; this
+// component of its D/2 goes to hres.  What does not depend on the sum is
+// loaded before it.
+template <class C>
+__device__ __forceinline__ void summer(DeltaSmemT<C> &S, int b, int c, int prev, int4 sl, int4 ln, float2 pk,
+                                       const StepParams &s, float &hres) {
+	const float2 xk = S.pos[sl.w];
 	const bool inList = (prev >= sl.x && prev < sl.x + ln.x) || (prev >= sl.y && prev < sl.y + ln.y) ||
 	                    (prev >= sl.z && prev < sl.z + ln.z);
-	if (!inList) return;
-	const float2 xk = S.pos[sl.w];
+	float x = finish_sum<C>(S, b ^ 1, c, hres);
+	const float o = __shfl_xor_sync(0x3u, x, 1);
+	const float2 xp = c == 0 ? make_float2(x, o) : make_float2(o, x);
 	const float rx = xp.x - xk.x, ry = xp.y - xk.y;
 	const float r2 = rx * rx + ry * ry;
-	if (r2 < s.h2) {
-		const float2 h = delta_half(xp, xk, r2, pk, s);
-		S.pos[prev] = make_float2(h.x + xp.x, h.y + xp.y);
-		hres = h;
-	}
+	const float h = comp(delta_half(xp, xk, r2, pk, s), c);
+	const bool in = inList && r2 < s.h2;
+	hres = in ? h : 0.0f;
+	*comp_of(&S.pos[prev], c) = in ? h + x : x;
 }
 
 // Process particles [p0, p1) (old numbers, or positions in AddParticle order
@@ -1977,8 +2057,9 @@ __device__ __forceinline__ unsigned long long relax_group(DeltaSmemT<C> &S, int 
 	const bool staged = stage_region<C>(S, R, Q, T, s, cellBase, tid);
 	const unsigned long long tStaged = global_ns();
 	bool pending = false;  // the previous particle still needs its sum (buffer ph ^ 1)
-	int ph = 0;
-	float2 hres = make_float2(0.0f, 0.0f);  // summer: D/2 of the pending particle's reserved pair
+	int ph = 0, prev = -1;  // prev: the pending particle's slot
+	float hres = 0.0f;  // summer lanes: this component of D/2 of the pending particle's reserved pair
+	const uint4 below = warps_below(warp);
 	for (int c0 = p0; c0 < p1; c0 += C::kPrefetch) {
 		const int c1 = min(p1, c0 + C::kPrefetch);
 		for (int k = c0 + tid; k < c1; k += kDT) {
@@ -1995,30 +2076,66 @@ __device__ __forceinline__ unsigned long long relax_group(DeltaSmemT<C> &S, int 
 			}
 		}
 		__syncthreads();
+		// A particle's inputs are loaded a phase ahead (kDirect: this thread's
+		// first list entry too), beside the arithmetic of the current one.
+		int4 slN = make_int4(0, 0, 0, -1), lnN = make_int4(0, 0, 0, 0);
+		float2 pkN = S.ppk[0];
+		int atN = -1;
+		if (staged) {
+			slN = S.pslot[0];
+			lnN = S.plen[0];
+			if (C::kDirect && warp < kP) atN = direct_slot<C>(slN, lnN, tid, 0);
+		}
 		for (int k = c0; k < c1; ++k) {
-			const float2 pk = S.ppk[k - c0];
 			if (staged) {
-				const int4 sl = S.pslot[k - c0], ln = S.plen[k - c0];
+				const int4 sl = slN, ln = lnN;
+				const float2 pk = pkN;
+				const int at0 = atN, kn = min(k + 1, c1 - 1) - c0;
+				slN = S.pslot[kn];
+				lnN = S.plen[kn];
+				pkN = S.ppk[kn];
 				if (C::kPipelined && sl.w >= 0 && ln.x + ln.y + ln.z <= DeltaSmemT<C>::kPass) {
 					const int b = (ph & 1) % DeltaSmemT<C>::kPhases;
+					const int pend = pending ? prev : -1;
 					if (warp < kP) {
-						produce<C>(S, b, sl, ln, pk, pending ? S.meta[b ^ 1].z : -1, s, tid);
-					} else if (pending && lane == 0) {
-						summer<C>(S, b, sl, ln, pk, s, hres);
+						if constexpr (C::kDirect) {
+							constexpr int kE = C::kChainW / kWarp;
+							if (ln.w <= kWarp) {
+								produce_direct<C, 1>(S, b, &at0, sl.w, pk, pend, below, s, tid);
+							} else {
+								int at[kE];
+								at[0] = at0;
+#pragma unroll
+								for (int i = 1; i < kE; ++i) at[i] = direct_slot<C>(sl, ln, tid, i);
+								if (ln.w <= 2 * kWarp)
+									produce_direct<C, 2>(S, b, at, sl.w, pk, pend, below, s, tid);
+								else
+									produce_direct<C, kE>(S, b, at, sl.w, pk, pend, below, s, tid);
+							}
+							atN = direct_slot<C>(slN, lnN, tid, 0);
+						} else {
+							produce<C>(S, b, sl, ln, pk, pend, s, tid);
+						}
+					} else if (pending && lane < 2) {
+						summer<C>(S, b, lane, prev, sl, ln, pk, s, hres);
 					}
 					__syncthreads();
+					prev = sl.w;
 					pending = true;
 					++ph;
 					continue;
 				}
+				if (C::kDirect && warp < kP) atN = direct_slot<C>(slN, lnN, tid, 0);
 				// Drain the pipeline, then relax this particle on the whole block.
-				if (C::kPipelined && pending && warp == kP && lane == 0) finish_particle<C>(S, (ph & 1) ^ 1, hres);
+				if (C::kPipelined && pending && warp == kP && lane < 2)
+					*comp_of(&S.pos[prev], lane) = finish_sum<C>(S, (ph & 1) ^ 1, lane, hres);
 				__syncthreads();
 				pending = false;
 				relax_particle<C>(S, sl, ln, pk, s, tid);
 				continue;
 			}
 			const int nc = S.pnc[k - c0], jk = S.pjk[k - c0];
+			const float2 pk = S.ppk[k - c0];
 			Region R1;
 			const int x = (nc - cellBase) % s.gx, y = (nc - cellBase) / s.gx;
 			R1.x0 = max(x - 1, 0);
@@ -2038,7 +2155,8 @@ __device__ __forceinline__ unsigned long long relax_group(DeltaSmemT<C> &S, int 
 		}
 		__syncthreads();
 	}
-	if (C::kPipelined && pending && warp == kP && lane == 0) finish_particle<C>(S, (ph & 1) ^ 1, hres);
+	if (C::kPipelined && pending && warp == kP && lane < 2)
+		*comp_of(&S.pos[prev], lane) = finish_sum<C>(S, (ph & 1) ^ 1, lane, hres);
 	__syncthreads();
 	if (staged) write_back_owned<C>(S, R, Q, tid);
 	return tStaged;

@@ -30,19 +30,19 @@ struct ViscLean {
 struct DeltaWide {
 	static constexpr int kWarps = 12, kStage = kDeltaStageCap, kChainW = 96, kPrefetch = 128, kMinBlocks = 1;
 	static constexpr int kRegion = kRegionCells;
-	static constexpr bool kPipelined = true, kShortEntry = true;
+	static constexpr bool kPipelined = true, kShortEntry = true, kDirect = true;
 };
 struct DeltaLean {
 	static constexpr int kWarps = 2, kStage = 1536, kChainW = 192, kPrefetch = 64, kMinBlocks = 8;
 	static constexpr int kRegion = kRegionCells;
-	static constexpr bool kPipelined = false, kShortEntry = false;
+	static constexpr bool kPipelined = false, kShortEntry = false, kDirect = false;
 };
 // Mid: pipelined, eight warps, two blocks per SM (mid-size scenes, where
 // more tasks run at once than one block per SM holds).
 struct DeltaMid {
 	static constexpr int kWarps = 8, kStage = kDeltaStageCap, kChainW = 128, kPrefetch = 128, kMinBlocks = 2;
 	static constexpr int kRegion = 256;
-	static constexpr bool kPipelined = true, kShortEntry = true;
+	static constexpr bool kPipelined = true, kShortEntry = true, kDirect = true;
 };
 // Small pipelined shapes for large scenes, where the sweep is bound by how
 // many tasks run at once rather than by one task's latency: two (tri) or
@@ -50,12 +50,12 @@ struct DeltaMid {
 struct DeltaTri {
 	static constexpr int kWarps = 3, kStage = 1536, kChainW = 256, kPrefetch = 64, kMinBlocks = 5;
 	static constexpr int kRegion = kRegionCells;
-	static constexpr bool kPipelined = true, kShortEntry = true;
+	static constexpr bool kPipelined = true, kShortEntry = true, kDirect = false;
 };
 struct DeltaQuad {
 	static constexpr int kWarps = 4, kStage = 1536, kChainW = 192, kPrefetch = 128, kMinBlocks = 4;
 	static constexpr int kRegion = kRegionCells;
-	static constexpr bool kPipelined = true, kShortEntry = true;
+	static constexpr bool kPipelined = true, kShortEntry = true, kDirect = false;
 };
 // Dense: pipelined, sixteen warps, one block per SM, a 12,288-entry stage,
 // for crowded states where a task's region (the bounding box of its
@@ -64,7 +64,7 @@ struct DeltaQuad {
 struct DeltaDense {
 	static constexpr int kWarps = 16, kStage = kDeltaDenseStageCap, kChainW = 96, kPrefetch = 128, kMinBlocks = 1;
 	static constexpr int kRegion = 400;
-	static constexpr bool kPipelined = true, kShortEntry = true;
+	static constexpr bool kPipelined = true, kShortEntry = true, kDirect = true;
 };
 // Delta shapes by index (sph_set_sweep_shape names them by warp count).
 constexpr int kDeltaShapes = 6;
