@@ -291,8 +291,8 @@ int sph_use_graphs(sph_sim *sim, int enable);
  * producer warps beside one summer warp; mid, quad and tri run several
  * blocks per SM; dense stages 12,288 entries per task, for crowded
  * states).  The lean ones
- * fit more tasks on an SM (the lean viscosity sweep runs five tasks per
- * block) for large scenes and many scenes.  Results do not depend on the
+ * fit more tasks on an SM (the lean viscosity sweep runs eighteen tasks
+ * per block) for large scenes and many scenes.  Results do not depend on the
  * shape.  sph_autotune times the
  * next update (step dt) from the current state for every shape and resident
  * block count per SM, keeps the fastest for each sweep, restores the state

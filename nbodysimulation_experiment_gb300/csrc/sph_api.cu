@@ -2039,7 +2039,7 @@ int sph_autotune(sph_sim *s, float dt, int *shape) {
 	if (rc) return rc;
 	SPH_CUDA(cudaStreamSynchronize(s->stream));
 	if (shape) {
-		shape[0] = s->viscLean ? ViscLean::kWarps : ViscWide::kWarps;
+		shape[0] = s->viscLean ? ViscLean::kName : ViscWide::kWarps;
 		shape[1] = s->viscBlocks;
 		shape[2] = delta_shape_warps(s->deltaShape);
 		shape[3] = s->deltaBlocks;
@@ -2049,7 +2049,7 @@ int sph_autotune(sph_sim *s, float dt, int *shape) {
 
 int sph_get_sweep_shape(sph_sim *s, int *shape) {
 	if (!s || !shape) return SPH_ERR_INVALID_ARGUMENT;
-	shape[0] = s->viscLean ? ViscLean::kWarps : ViscWide::kWarps;
+	shape[0] = s->viscLean ? ViscLean::kName : ViscWide::kWarps;
 	shape[1] = s->viscBlocks;
 	shape[2] = delta_shape_warps(s->deltaShape);
 	shape[3] = s->deltaBlocks;
@@ -2058,7 +2058,7 @@ int sph_get_sweep_shape(sph_sim *s, int *shape) {
 
 int sph_set_sweep_shape(sph_sim *s, const int *shape) {
 	if (!s || !shape) return SPH_ERR_INVALID_ARGUMENT;
-	const bool vOk = shape[0] == ViscLean::kWarps || shape[0] == ViscWide::kWarps;
+	const bool vOk = shape[0] == ViscLean::kName || shape[0] == ViscWide::kWarps;
 	int dShape = -1;
 	for (int k = 0; k < kDeltaShapes; ++k)
 		if (shape[2] == delta_shape_warps(k)) dShape = k;
@@ -2066,7 +2066,7 @@ int sph_set_sweep_shape(sph_sim *s, const int *shape) {
 	if (!vOk || !dOk || shape[1] < 1 || shape[3] < 1 || shape[1] > (1 << 20) || shape[3] > (1 << 20))
 		return SPH_ERR_INVALID_ARGUMENT;
 	SPH_CUDA(cudaStreamSynchronize(s->stream));
-	s->viscLean = shape[0] == ViscLean::kWarps;
+	s->viscLean = shape[0] == ViscLean::kName;
 	s->viscBlocks = shape[1];
 	s->deltaShape = dShape;
 	s->deltaBlocks = shape[3];
@@ -2083,7 +2083,7 @@ int sph_set_adaptive_shapes(sph_sim *s, int enable) {
 int sph_last_sweep_shape(sph_sim *s, int *shape) {
 	if (!s || !shape) return SPH_ERR_INVALID_ARGUMENT;
 	if (s->runViscLean < 0) return sph_get_sweep_shape(s, shape);
-	shape[0] = s->runViscLean ? ViscLean::kWarps : ViscWide::kWarps;
+	shape[0] = s->runViscLean ? ViscLean::kName : ViscWide::kWarps;
 	shape[1] = s->runViscBlocks;
 	shape[2] = delta_shape_warps(s->runDeltaShape);
 	shape[3] = s->runDeltaBlocks;

@@ -316,8 +316,20 @@ __device__ __forceinline__ void visc_pair(uint32_t at, float2 n, float o, float2
 __device__ __forceinline__ uint32_t shared_addr(const void *p) {
 	return (uint32_t)__cvta_generic_to_shared(p);
 }
-__device__ __forceinline__ float2 vel_at(const float2 *vel, int off) {
-	return *reinterpret_cast<const float2 *>(reinterpret_cast<const char *>(vel) + off);
+// Loads of the chains by shared-memory address, in program order with the
+// stores of visc_pair.
+__device__ __forceinline__ float2 lds2(uint32_t at) {
+	float2 v;
+	asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(at) : "memory");
+	return v;
+}
+__device__ __forceinline__ float4 lds4(uint32_t at) {
+	float4 v;
+	asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
+	             : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+	             : "r"(at)
+	             : "memory");
+	return v;
 }
 
 // The ordered chain over the len buffered pairs G[0..len) (byte offset of the
@@ -335,34 +347,35 @@ __device__ __forceinline__ float2 vel_at(const float2 *vel, int off) {
 // loads between every two pairs; ten dependent operations alone take 47.
 __device__ __forceinline__ void visc_chain(const float2 *vel, const float4 *G, const float4 *idle, int len, int n,
                                            float2 &vi, float sigma, float beta, float hdt) {
-	const float4 *src = len > 0 ? G : idle;
-	const int last = max(len - 1, 0);
 	const uint32_t base = shared_addr(vel);
+	uint32_t at = shared_addr(len > 0 ? G : idle);
+	const uint32_t end = at + 16u * (uint32_t)max(len - 1, 0);
 	float4 g[4], h[4];
 	float2 v[4], w[4];
 #pragma unroll
-	for (int u = 0; u < 4; ++u) g[u] = src[min(u, last)];
+	for (int u = 0; u < 4; ++u) g[u] = lds4(min(at + 16u * u, end));
 #pragma unroll
-	for (int u = 0; u < 4; ++u) v[u] = vel_at(vel, __float_as_int(g[u].x));
+	for (int u = 0; u < 4; ++u) v[u] = lds2(base + __float_as_uint(g[u].x));
 #pragma unroll
-	for (int u = 0; u < 4; ++u) h[u] = src[min(4 + u, last)];
+	for (int u = 0; u < 4; ++u) h[u] = lds4(min(at + 64u + 16u * u, end));
 	for (int q = 0; q < n; q += 8) {
+		at += 128u;
 #pragma unroll
-		for (int u = 0; u < 4; ++u) w[u] = vel_at(vel, __float_as_int(h[u].x));
+		for (int u = 0; u < 4; ++u) w[u] = lds2(base + __float_as_uint(h[u].x));
 #pragma unroll
 		for (int u = 0; u < 4; ++u)
 			visc_pair(base + __float_as_uint(g[u].x), make_float2(g[u].y, g[u].z), g[u].w, v[u], vi, sigma, beta, hdt,
 			          q + u < len);
 #pragma unroll
-		for (int u = 0; u < 4; ++u) g[u] = src[min(q + 8 + u, last)];
+		for (int u = 0; u < 4; ++u) g[u] = lds4(min(at + 16u * u, end));
 #pragma unroll
 		for (int u = 0; u < 4; ++u)
 			visc_pair(base + __float_as_uint(h[u].x), make_float2(h[u].y, h[u].z), h[u].w, w[u], vi, sigma, beta, hdt,
 			          q + 4 + u < len);
 #pragma unroll
-		for (int u = 0; u < 4; ++u) v[u] = vel_at(vel, __float_as_int(g[u].x));
+		for (int u = 0; u < 4; ++u) v[u] = lds2(base + __float_as_uint(g[u].x));
 #pragma unroll
-		for (int u = 0; u < 4; ++u) h[u] = src[min(q + 12 + u, last)];
+		for (int u = 0; u < 4; ++u) h[u] = lds4(min(at + 64u + 16u * u, end));
 	}
 }
 
@@ -425,7 +438,7 @@ __device__ __forceinline__ void visc_wave(ViscSmemT<C> &S, int k, int cnt, int o
 	}
 	float2 vm[3];
 #pragma unroll
-	for (int u = 0; u < 3; ++u) vm[u] = vel_at(S.vel, __float_as_int(gm[u].x));
+	for (int u = 0; u < 3; ++u) vm[u] = lds2(base + __float_as_uint(gm[u].x));
 #pragma unroll
 	for (int u = 0; u < 3; ++u)
 		visc_pair(base + __float_as_uint(gm[u].x), make_float2(gm[u].y, gm[u].z), gm[u].w, vm[u], vi, s.sigma, s.beta,
@@ -538,170 +551,300 @@ __global__ void __launch_bounds__(C::kWarps * kWarp, C::kMinBlocks) k_viscosity(
 // ---------------------------------------------------------------------------
 // Viscosity sweep, many chains per block (the lean shape, ViscLean): the
 // same tasks, waits and arithmetic as k_viscosity, laid out for throughput.
-// A block holds kSlots tasks at once.  Lane s of warp 0 runs the ordered
-// velocity chain of slot s's current particle (the slots' chains share one
-// instruction stream), while producer warp 1 + (s % kProd) looks after slot
-// s: it claims a task, polls the task's earlier conflicting tasks (without
-// blocking), stages the velocities of its 3x3 block, computes the pair
-// geometry of the slot's next particle (positions, which this pass does not
-// change, are read through L1), and writes the velocities back and releases
-// the task when its chain is done.  The block advances in phases: one
-// particle per running slot per phase.
+// A block holds kSlots tasks at once.  The lanes of kChains chain warps run the
+// slots' ordered velocity chains (those of a warp share one instruction
+// stream), and a producer warp serves each slot: it claims a task, waits for
+// the task's earlier conflicting ones, stages the velocities of its 3x3 block,
+// holds the block's positions (which this pass does not change) in registers,
+// and keeps the pair geometry ahead of the chain in two buffers; when the chain
+// has taken the task's last particle it writes the velocities back and releases
+// the task.
+// The slots are decoupled: a producer publishes a segment of a particle's pairs
+// (ready), the chain lane takes it when its last one ends and says so (taken);
+// a particle with more pairs than a buffer holds comes in several segments.
+// A chain warp runs eight pairs at a time and its lanes change segments between
+// those, so no slot waits for another's longer list or for another's staging.
+// (In block-wide phases of one particle each, every phase took as long as the
+// longest of its chains, and longer still when some slot changed its task:
+// 11,700 cycles per particle on the 1M block against 7,400 alone.)  Blocks of
+// cells with more than kVelCap particles run from global memory on their
+// producer warp (slot_far_task).
+// Eighteen slots and two chain warps: sixteen or twenty slots, one or four
+// chain warps measured 0-9% slower (a block of more than 20 warps is left 80
+// registers a thread).  A turn of the chain loop takes ~600 cycles for twelve
+// pairs, ~160 more when a lane changes segments.  Per update, the same shape in
+// block-wide phases first: 1M block 2.60 -> 2.19 ms, 128 scenes 6.42 -> 4.53.
+struct ViscDesc {
+	int len;    // pairs of the segment
+	int own;    // byte offset of the particle's velocity + kSegFirst, kSegLast
+	float sigma, beta, hdt;
+	int pad[3];
+};
+constexpr int kSegFirst = 1, kSegLast = 2;
 template <class C>
 struct ViscSlotT {
-	float2 vel[kStageCap];    // velocities of the 3x3 block, list order
-	float4 geo[2][C::kGeom];  // per buffer: in-range pairs (byte offset into vel, unit vector, 1 - q) of one particle
+	float2 vel[C::kVelCap];   // velocities of the 3x3 block, list order
+	float4 geo[2][C::kGeom];  // per buffer: in-range pairs (byte offset into vel, unit vector, 1 - q) of one segment
 	float4 pad;               // consecutive slots start 16 bytes apart in the bank space
 };
 template <class C>
 struct ViscMultiSmemT {
 	ViscSlotT<C> slot[C::kSlots];
 	float4 idle;  // the entry of a chain without pairs
+	ViscDesc desc[C::kSlots][2];
 	int segStart[C::kSlots][9], segOff[C::kSlots][9];
-	int state[C::kSlots], task[C::kSlots], first[C::kSlots], cnt[C::kSlots], own[C::kSlots], L[C::kSlots],
-	    k[C::kSlots], cell[C::kSlots], claim[C::kSlots];
-	int m[C::kSlots][2];
-	float h2[C::kSlots], invH[C::kSlots], sigma[C::kSlots], beta[C::kSlots], hdt[C::kSlots];
-	unsigned long long waitSince[C::kSlots];
-	int exhausted;  // no tasks left to claim
-	int aborted;    // the abort flag was seen set
+	uint32_t ready[C::kSlots], taken[C::kSlots];  // segments published by the producer, finished by the chain
+	int exited;  // producers that found no more tasks
 };
 
 namespace {
 
-enum : int { kSlotFree = 0, kSlotWait = 1, kSlotStaged = 2, kSlotRun = 3, kSlotDone = 4 };
-
-// Pair geometry of particle k of slot s (one warp): in-range pairs in list
-// order (sph.h:497-505), compacted first, then the square roots and
-// divisions over the dense list.
-template <class C>
-__device__ __forceinline__ void slot_geometry(ViscMultiSmemT<C> &S, int s, int k, const Particles &P, int lane) {
-	const int buf = k & 1;
-	float4 *G = S.slot[s].geo[buf];
-	int segStart[9], segOff[9];
-#pragma unroll
-	for (int q = 0; q < 9; ++q) {
-		segStart[q] = S.segStart[s][q];
-		segOff[q] = S.segOff[s][q];
-	}
-	const int L = S.L[s];
-	const float h2 = S.h2[s], invH = S.invH[s];
-	const float2 xi = __ldg(&P.pos[S.first[s] + k]);
-	int m = 0;
-	for (int b0 = 0; b0 < L; b0 += 4 * kWarp) {
-		float2 xj[4];
-#pragma unroll
-		for (int u = 0; u < 4; ++u) {
-			const int e = b0 + u * kWarp + lane;
-			xj[u] = e < L ? __ldg(&P.pos[seg_src<9>(e, segOff, segStart)]) : make_float2(0.f, 0.f);
-		}
-#pragma unroll
-		for (int u = 0; u < 4; ++u) {
-			const int e = b0 + u * kWarp + lane;
-			const float rx = xj[u].x - xi.x, ry = xj[u].y - xi.y;
-			const float r2 = rx * rx + ry * ry;
-			const bool in = e < L && r2 < h2;
-			const unsigned mask = __ballot_sync(kFull, in);
-			const int at = m + __popc(mask & lanemask_lt());
-			if (in && at < C::kGeom) G[at] = make_float4(__int_as_float(8 * e), rx, ry, r2);
-			m += __popc(mask);
-		}
-	}
-	__syncwarp();
-	const int mm = min(m, C::kGeom);
-	for (int q = lane; q < mm; q += kWarp) {
-		const float4 g = G[q];
-		float r;  // Vec2Length(Rij) == rij
-		const float inv = root_and_inverse(g.w, r);
-		const float qq = r * invH;
-		G[q] = make_float4(g.x, g.y * inv, g.z * inv, 1.0f - qq);
-	}
-	if (lane == 0) S.m[s][buf] = m;
+__device__ __forceinline__ uint32_t ld_acquire_cta(const uint32_t *p) {
+	uint32_t v;
+	asm volatile("ld.acquire.cta.shared.u32 %0, [%1];" : "=r"(v) : "r"(shared_addr(p)) : "memory");
+	return v;
+}
+__device__ __forceinline__ void st_release_cta(uint32_t *p, uint32_t v) {
+	asm volatile("st.release.cta.shared.u32 [%0], %1;" ::"r"(shared_addr(p)), "r"(v) : "memory");
 }
 
-// Claim the next task into slot s (one warp).  Returns false when none is
-// left.
+// Bounded wait of a producer warp until the chain has finished `count`
+// segments of slot s (a segment takes some 5 us).  False when it gave up, with
+// kErrTimeout and the abort flag raised.  Polled every 500 ns: more often, the
+// polling slowed the chains (2.67 against 2.88 ms on the 1M block).
+constexpr uint32_t kTakenPolls = 1u << 22;
 template <class C>
-__device__ __forceinline__ bool slot_claim(ViscMultiSmemT<C> &S, int s, const SimTables &T, int nLive, int lane) {
-	int i = 0;
-	if (lane == 0) i = atomicAdd(&T.taskCounter[0], 1);
-	i = __shfl_sync(kFull, i, 0);
-	if (i >= nLive) return false;
-	const int t = T.liveTask[i];
-	const int c = T.taskCell[t];
-	const SceneDev &sc = T.scenes[T.sceneOfCell[c]];
-	const int base = sc.cellBase, gx = sc.p.gx, gy = sc.p.gy;
-	const int cx = (c - base) % gx, cy = (c - base) / gx;
-	// Segments of the 3x3 block in list order (lanes 0..8, then a scan).
-	int st = 0, nn = 0;
-	if (lane < 9) {
-		const int x = cx + lane % 3 - 1, y = cy + lane / 3 - 1;
-		if (x >= 0 && x < gx && y >= 0 && y < gy) {
-			const int c2 = base + y * gx + x;
-			st = T.cellStart[c2];
-			nn = T.cellCount[c2];
-		}
+__device__ __forceinline__ bool slot_taken(ViscMultiSmemT<C> &S, int s, uint32_t count, const SimTables &T) {
+	for (uint32_t it = 0; it < kTakenPolls; ++it) {
+		const bool ok = (int)(ld_acquire_cta(&S.taken[s]) - count) >= 0;
+		if (__all_sync(kFull, ok)) return true;
+		__nanosleep(500);
 	}
-	int incl = nn;
-#pragma unroll
-	for (int o = 1; o < 16; o <<= 1) {
-		const int v = __shfl_up_sync(kFull, incl, o);
-		if (lane >= o) incl += v;
+	if ((threadIdx.x & (kWarp - 1)) == 0) {
+		atomicOr(T.error, kErrTimeout);
+		atomicExch(T.abort, 1u);
 	}
-	if (lane < 9) {
-		S.segStart[s][lane] = st;
-		S.segOff[s][lane] = incl - nn;
-	}
-	const int L = __shfl_sync(kFull, incl, 8);
-	const int own = __shfl_sync(kFull, incl - nn, 4);
-	if (lane == 0) {
-		S.task[s] = t;
-		S.claim[s] = i;
-		S.cell[s] = c;
-		S.first[s] = T.cellStart[c];
-		S.cnt[s] = T.cellCount[c];
-		S.own[s] = own;
-		S.L[s] = L;
-		S.h2[s] = sc.p.h2;
-		S.invH[s] = sc.p.invH;
-		S.sigma[s] = sc.p.sigma;
-		S.beta[s] = sc.p.beta;
-		S.hdt[s] = 0.5f * sc.p.dt;
-		S.state[s] = kSlotWait;
-		S.waitSince[s] = global_ns();
-	}
-	stamp(T, 0, t, 0, lane);
+	return false;
+}
+
+// A producer warp's open segment.
+struct ViscSegment {
+	uint32_t seq;  // segments published so far: this one's number
+	int m;         // pairs compacted into it
+	int own;       // the particle's velocity offset, + kSegFirst on its first segment
+};
+
+// Publish the open segment (one warp): the square roots and divisions over
+// its compacted entries (byte offset, r, r^2), then its descriptor; wait until
+// the next buffer is free.  False when the wait gave up.
+template <class C>
+__device__ __forceinline__ bool slot_publish(ViscMultiSmemT<C> &S, int s, ViscSegment &g, bool last, float invH,
+                                             const StepParams &p, const SimTables &T, int lane) {
+	float4 *G = S.slot[s].geo[g.seq & 1u];
 	__syncwarp();
+	for (int q = lane; q < g.m; q += kWarp) {
+		const float4 e = G[q];
+		float r;  // Vec2Length(Rij) == rij
+		const float inv = root_and_inverse(e.w, r);
+		const float qq = r * invH;
+		G[q] = make_float4(e.x, e.y * inv, e.z * inv, 1.0f - qq);
+	}
+	if (lane == 0) {
+		ViscDesc &d = S.desc[s][g.seq & 1u];
+		d.len = g.m;
+		d.own = g.own + (last ? kSegLast : 0);
+		d.sigma = p.sigma;
+		d.beta = p.beta;
+		d.hdt = 0.5f * p.dt;
+	}
+	__syncwarp();
+	++g.seq;
+	if (lane == 0) st_release_cta(&S.ready[s], g.seq);
+	g.m = 0;
+	g.own &= ~kSegFirst;
+	// The next buffer held segment seq - 2.
+	return g.seq < 2 || slot_taken<C>(S, s, g.seq - 1, T);
+}
+
+// One batch of 32 list entries (one per lane, at byte offset `off` of the
+// block's velocities, position xj) of the particle at xi: the in-range ones
+// (sph.h:497-505) join the segment in list order.
+template <class C>
+__device__ __forceinline__ bool slot_entries(ViscMultiSmemT<C> &S, int s, ViscSegment &g, int off, float2 xj, bool valid,
+                                             float2 xi, float h2, float invH, const StepParams &p, const SimTables &T,
+                                             int lane) {
+	const float rx = xj.x - xi.x, ry = xj.y - xi.y;
+	const float r2 = rx * rx + ry * ry;
+	const bool in = valid && r2 < h2;
+	const unsigned mask = __ballot_sync(kFull, in);
+	const int n = __popc(mask);
+	if (g.m + n > C::kGeom && !slot_publish<C>(S, s, g, false, invH, p, T, lane)) return false;
+	if (in) S.slot[s].geo[g.seq & 1u][g.m + __popc(mask & lanemask_lt())] = make_float4(__int_as_float(off), rx, ry, r2);
+	g.m += n;
 	return true;
 }
 
-// One non-blocking poll of slot s's earlier conflicting tasks (cells of the
-// scene at most two apart, as k_viscosity).  True when all are done.
+// A chain warp: lane l runs the segments of slot first + l in the order
+// published, 3 U pairs per turn of the loop (U = kChainGroup) in three groups
+// with a register set each: while a group runs, the next one's partner
+// velocities and the next but one's geometry load.  Within a turn a lane's
+// next turn is settled (this segment, the next one if this ends here and it is
+// ready, or nothing), so its geometry is on its way before the turn ends; what
+// depends on the finished pairs (the velocity to store, the next particle's
+// own and its first partners') follows at the end, in the turns where a lane
+// changes.
+constexpr int kChainGroup = 4;
 template <class C>
-__device__ __forceinline__ bool slot_ready(ViscMultiSmemT<C> &S, int s, const SimTables &T, int lane) {
-	const int t = S.task[s], c = S.cell[s];
-	const SceneDev &sc = T.scenes[T.sceneOfCell[c]];
-	const int base = sc.cellBase, gx = sc.p.gx, gy = sc.p.gy;
-	const int cx = (c - base) % gx, cy = (c - base) / gx;
-	bool pending = false;
-	const int x = cx + lane % 5 - 2, y = cy + lane / 5 - 2;
-	if (lane < 25 && lane != 12 && x >= 0 && x < gx && y >= 0 && y < gy) {
-		const int c2 = base + y * gx + x;
-		const int r2 = T.taskOfCell[c2];
-		if (r2 < t && T.cellCount[c2] > 0) pending = ld_acquire(&T.done[r2]) == 0u;
+__device__ __forceinline__ void slot_chains(ViscMultiSmemT<C> &S, int first, int lane) {
+	constexpr int kLanes = C::kSlots / C::kChains, U = kChainGroup;
+	const bool mine = lane < kLanes;
+	const int s = first + (mine ? lane : 0);
+	const uint32_t base = shared_addr(S.slot[s].vel), geo = shared_addr(S.slot[s].geo[0]);
+	const uint32_t idle = shared_addr(&S.idle);
+	uint32_t at = idle, end = idle;  // a turn's first entry, the segment's last
+	int left = 0, own = 0;           // pairs left at the start of a turn
+	uint32_t seq = 0;                // segments begun
+	bool active = false;
+	float2 vi = make_float2(0.f, 0.f);
+	float sigma = 0.f, beta = 0.f, hdt = 0.f;
+	float4 ga[U], gb[U], gc[U];
+	float2 va[U], vb[U], vc[U];
+	auto geometry = [&](float4(&g)[U], uint32_t from, uint32_t to) {
+#pragma unroll
+		for (int u = 0; u < U; ++u) g[u] = lds4(min(from + 16u * u, to));
+	};
+	auto partners = [&](float2(&v)[U], const float4(&g)[U]) {
+#pragma unroll
+		for (int u = 0; u < U; ++u) v[u] = lds2(base + __float_as_uint(g[u].x));
+	};
+	auto pairs = [&](const float4(&g)[U], const float2(&v)[U], int first) {
+#pragma unroll
+		for (int u = 0; u < U; ++u)
+			visc_pair(base + __float_as_uint(g[u].x), make_float2(g[u].y, g[u].z), g[u].w, v[u], vi, sigma, beta, hdt,
+			          first + u < left);
+	};
+	geometry(ga, at, end);
+	geometry(gb, at, end);
+	partners(va, ga);
+	for (uint32_t it = 0;; ++it) {
+		if ((it & 15u) == 0u && !__any_sync(kFull, active)) {
+			if (*(volatile int *)&S.exited == C::kSlots) break;
+			__nanosleep(64);
+		}
+		uint32_t rdy;
+		asm volatile("ld.relaxed.cta.shared.u32 %0, [%1];" : "=r"(rdy) : "r"(shared_addr(&S.ready[s])) : "memory");
+		partners(vb, gb);
+		geometry(gc, at + 32u * U, end);
+		pairs(ga, va, 0);
+		const bool fin = left <= 3 * U, sw = mine && fin && (int)(rdy - seq) > 0;
+		const bool event = __any_sync(kFull, sw || (fin && active));
+		int leftN = left - 3 * U;
+		float4 n4 = make_float4(0.f, 0.f, 0.f, 0.f);
+		float nHdt = 0.0f;
+		at += 48u * U;
+		if (event) {
+			__threadfence_block();  // ready before the segment it announces
+			const uint32_t desc = shared_addr(&S.desc[s][seq & 1u]);
+			n4 = lds4(desc);
+			nHdt = lds2(desc + 16u).x;
+			if (fin) {
+				leftN = sw ? __float_as_int(n4.x) : 0;
+				at = leftN > 0 ? geo + (seq & 1u) * (uint32_t)sizeof(S.slot[0].geo[0]) : idle;
+				end = at + 16u * (uint32_t)max(leftN - 1, 0);
+			}
+		}
+		partners(vc, gc);
+		geometry(ga, at, end);
+		pairs(gb, vb, U);
+		partners(va, ga);
+		geometry(gb, at + 16u * U, end);
+		pairs(gc, vc, 2 * U);
+		if (event) {
+			const int done = fin && active ? 1 : 0;
+			asm volatile(
+			    "{\n"
+			    ".reg .pred p, q;\n"
+			    "setp.ne.s32 q, %0, 0;\n"
+			    "setp.ne.s32 p, %1, 0;\n"
+			    "@p st.shared.v2.f32 [%2], {%3, %4};\n"
+			    "@q st.release.cta.shared.u32 [%5], %6;\n"
+			    "}\n" ::"r"(done),
+			    "r"(done && (own & kSegLast) ? 1 : 0), "r"(base + (own & ~7)), "f"(vi.x), "f"(vi.y),
+			    "r"(shared_addr(&S.taken[s])), "r"(seq)
+			    : "memory");
+			active = fin ? sw : active;
+			own = sw ? __float_as_int(n4.y) : own;
+			sigma = sw ? n4.z : sigma;
+			beta = sw ? n4.w : beta;
+			hdt = sw ? nHdt : hdt;
+			const float2 nv = lds2(base + (own & ~7));
+			if (sw && (own & kSegFirst)) vi = nv;
+			seq += sw ? 1u : 0u;
+			partners(va, ga);
+		}
+		left = leftN;
 	}
-	return !__any_sync(kFull, pending);
 }
 
+// A task whose 3x3 block outgrows the slot, on its producer warp, velocities
+// in global memory: per batch of 32 list entries every lane loads and
+// evaluates its own, then all lanes run the ordered chain over the in-range
+// ones (a partner occurs once per list, so its velocity may be loaded before
+// the chain reaches it) and each lane stores its partner's new velocity.
 template <class C>
-__device__ __forceinline__ void slot_copy_vel(ViscMultiSmemT<C> &S, int s, const Particles &P, int lane, bool in) {
+__device__ __noinline__ void slot_far_task(ViscMultiSmemT<C> &S, int s, int L, int first, int cnt, const StepParams &p,
+                                           float2 *vel, const float2 *__restrict__ pos, int lane) {
 	int segStart[9], segOff[9];
 #pragma unroll
 	for (int q = 0; q < 9; ++q) {
 		segStart[q] = S.segStart[s][q];
 		segOff[q] = S.segOff[s][q];
 	}
-	const int L = S.L[s];
+	const float hdt = 0.5f * p.dt;
+	for (int k = 0; k < cnt; ++k) {
+		const float2 xi = __ldg(&pos[first + k]);
+		float2 vi = __ldcg(&vel[first + k]);
+		for (int b0 = 0; b0 < L; b0 += kWarp) {
+			const int e = b0 + lane;
+			const int j = e < L ? seg_src<9>(e, segOff, segStart) : first;
+			const float2 xj = __ldg(&pos[j]);
+			float2 vj = __ldcg(&vel[j]);
+			const float rx = xj.x - xi.x, ry = xj.y - xi.y;
+			const float r2 = rx * rx + ry * ry;
+			const bool in = e < L && r2 < p.h2;
+			float r;
+			const float inv = root_and_inverse(r2, r);
+			const float nx = rx * inv, ny = ry * inv, o = 1.0f - r * p.invH;
+			bool moved = false;
+			for (unsigned mask = __ballot_sync(kFull, in); mask; mask &= mask - 1) {
+				const int t = __ffs(mask) - 1;
+				const float tx = __shfl_sync(kFull, nx, t), ty = __shfl_sync(kFull, ny, t), to = __shfl_sync(kFull, o, t);
+				const float wx = __shfl_sync(kFull, vj.x, t), wy = __shfl_sync(kFull, vj.y, t);
+				const float uu = (vi.x - wx) * tx + (vi.y - wy) * ty;
+				if (uu > 0.0f) {
+					const float f = to * (p.sigma * uu + p.beta * (uu * uu));
+					const float ix = (f * tx) * hdt;
+					const float iy = (f * ty) * hdt;
+					vi.x = vi.x - ix;
+					vi.y = vi.y - iy;
+					if (lane == t) {
+						vj = make_float2(ix + wx, iy + wy);
+						moved = true;
+					}
+				}
+			}
+			if (moved) __stcg(&vel[j], vj);
+		}
+		__syncwarp();
+		if (lane == 0) __stcg(&vel[first + k], vi);
+		__syncwarp();
+	}
+}
+
+// Copy the block's velocities between the slot and global memory (one warp).
+template <class C>
+__device__ __forceinline__ void slot_copy_vel(ViscMultiSmemT<C> &S, int s, int L, const int (&segStart)[9],
+                                              const int (&segOff)[9], const Particles &P, int lane, bool in) {
 	float2 *V = S.slot[s].vel;
 	for (int b0 = 0; b0 < L; b0 += 4 * kWarp) {
 		if (in) {
@@ -726,150 +869,156 @@ __device__ __forceinline__ void slot_copy_vel(ViscMultiSmemT<C> &S, int s, const
 	}
 }
 
-// The producer warp's turn for slot s in one phase.
+// Producer warp of slot s: tasks until none is left.
 template <class C>
-__device__ __forceinline__ void slot_produce(ViscMultiSmemT<C> &S, int s, const Particles &P, const SimTables &T,
-                                             int nLive, int lane) {
-	int state = S.state[s];
-	if (state == kSlotDone) {
-		// Chain finished: write the block's velocities back and release.
-		slot_copy_vel<C>(S, s, P, lane, false);
-		__threadfence();
-		__syncwarp();
-		stamp(T, 0, S.task[s], 3, lane);
-		if (lane == 0) {
-			if (S.claim[s] != T.hold[0]) st_release(&T.done[S.task[s]], 1u);
-			S.state[s] = kSlotFree;
-		}
-		__syncwarp();
-		state = kSlotFree;
-	}
-	if (state == kSlotFree) {
-		if (__shfl_sync(kFull, S.exhausted, 0)) return;
-		if (!slot_claim<C>(S, s, T, nLive, lane)) {
-			if (lane == 0) S.exhausted = 1;
-			return;
-		}
-		state = kSlotWait;
-	}
-	if (state == kSlotWait) {
-		if (!slot_ready<C>(S, s, T, lane)) {
-			if (lane == 0 && global_ns() - S.waitSince[s] > T.waitLimitNs) {
-				atomicOr(T.error, kErrTimeout);
-				atomicExch(T.abort, 1u);
+__device__ __forceinline__ void slot_producer(ViscMultiSmemT<C> &S, int s, const Particles &P, const SimTables &T,
+                                              int nLive, int lane) {
+	ViscSegment seg{0u, 0, 0};
+	for (;;) {
+		int i = 0;
+		if (lane == 0) i = atomicAdd(&T.taskCounter[0], 1);
+		i = __shfl_sync(kFull, i, 0);
+		if (i >= nLive) return;
+		const int t = T.liveTask[i];
+		stamp(T, 0, t, 0, lane);
+		const int c = T.taskCell[t];
+		const SceneDev &sc = T.scenes[T.sceneOfCell[c]];
+		const int base = sc.cellBase, gx = sc.p.gx, gy = sc.p.gy;
+		const int cx = (c - base) % gx, cy = (c - base) / gx;
+		const float h2 = sc.p.h2, invH = sc.p.invH;
+		// Segments of the 3x3 block in list order (lanes 0..8, then a scan).
+		int st = 0, nn = 0;
+		if (lane < 9) {
+			const int x = cx + lane % 3 - 1, y = cy + lane / 3 - 1;
+			if (x >= 0 && x < gx && y >= 0 && y < gy) {
+				const int c2 = base + y * gx + x;
+				st = T.cellStart[c2];
+				nn = T.cellCount[c2];
 			}
-			return;
 		}
-		if (S.L[s] > kStageCap) {
-			// The block does not fit: flag it and release the task untouched.
-			if (lane == 0) {
-				atomicOr(T.error, kErrStageOverflow);
-				st_release(&T.done[S.task[s]], 1u);
-				S.state[s] = kSlotFree;
-			}
-			__syncwarp();
-			return;
+		int incl = nn;
+#pragma unroll
+		for (int o = 1; o < 16; o <<= 1) {
+			const int v = __shfl_up_sync(kFull, incl, o);
+			if (lane >= o) incl += v;
 		}
-		stamp(T, 0, S.task[s], 1, lane);
-		slot_copy_vel<C>(S, s, P, lane, true);
-		slot_geometry<C>(S, s, 0, P, lane);
-		if (lane == 0) S.state[s] = kSlotStaged;
+		if (lane < 9) {
+			S.segStart[s][lane] = st;
+			S.segOff[s][lane] = incl - nn;
+		}
+		const int L = __shfl_sync(kFull, incl, 8);
+		const int own = __shfl_sync(kFull, incl - nn, 4);
+		const int first = __shfl_sync(kFull, st, 4), cnt = __shfl_sync(kFull, nn, 4);
 		__syncwarp();
-		return;
-	}
-	if (state == kSlotRun) {
-		const int k = S.k[s];
-		if (k + 1 < S.cnt[s]) slot_geometry<C>(S, s, k + 1, P, lane);
-	}
-}
-
-// The chain of slot s's current particle (lane s of warp 0; `running` is the
-// mask of the lanes that run one).
-template <class C>
-__device__ __forceinline__ void slot_chain(ViscMultiSmemT<C> &S, int s, unsigned running, const Particles &P) {
-	const int k = S.k[s], buf = k & 1, m = S.m[s][buf];
-	const int own = S.own[s] + k;
-	float2 *V = S.slot[s].vel;
-	const float sigma = S.sigma[s], beta = S.beta[s], hdt = S.hdt[s];
-	const uint32_t base = shared_addr(V);
-	float2 vi = V[own];
-	if (m > C::kGeom) {
-		// More in-range pairs than the geometry buffer holds: the same pair
-		// geometry (sph.h:497-505), computed here in list order.
+		// The block's positions do not depend on the earlier tasks.
+		float2 px[C::kRegEntries];
+		const bool regs = L <= C::kRegEntries * kWarp;
 		int segStart[9], segOff[9];
 #pragma unroll
 		for (int q = 0; q < 9; ++q) {
 			segStart[q] = S.segStart[s][q];
 			segOff[q] = S.segOff[s][q];
 		}
-		const int L = S.L[s];
-		const float h2 = S.h2[s], invH = S.invH[s];
-		const float2 xi = __ldg(&P.pos[S.first[s] + k]);
-		for (int e = 0; e < L; ++e) {
-			const float2 xj = __ldg(&P.pos[seg_src<9>(e, segOff, segStart)]);
-			const float rx = xj.x - xi.x, ry = xj.y - xi.y;
-			const float r2 = rx * rx + ry * ry;
-			if (!(r2 < h2)) continue;
-			const float r = sqrtf(r2);
-			const float qq = r * invH;
-			float len = r;
-			if (len == 0.0f) len = 1.0f;
-			const float inv = 1.0f / len;
-			visc_pair(base + 8u * e, make_float2(rx * inv, ry * inv), 1.0f - qq, V[e], vi, sigma, beta, hdt);
+		if (regs) {
+#pragma unroll
+			for (int r = 0; r < C::kRegEntries; ++r) {
+				const int e = r * kWarp + lane;
+				px[r] = e < L ? __ldg(&P.pos[seg_src<9>(e, segOff, segStart)]) : make_float2(3.0e38f, 3.0e38f);
+			}
 		}
+		// Wait for earlier tasks of the scene within Chebyshev distance 2.
+		{
+			const uint32_t *flag = nullptr;
+			const int x = cx + lane % 5 - 2, y = cy + lane / 5 - 2;
+			if (lane < 25 && lane != 12 && x >= 0 && x < gx && y >= 0 && y < gy) {
+				const int c2 = base + y * gx + x;
+				const int r2 = T.taskOfCell[c2];
+				if (r2 < t && T.cellCount[c2] > 0) flag = &T.done[r2];
+			}
+			warp_wait(flag, T.abort, T.error, T.waitLimitNs);
+		}
+		if (__shfl_sync(kFull, lane == 0 ? ld_acquire(T.abort) : 0u, 0) != 0u) return;
+		stamp(T, 0, t, 1, lane);
+		if (L > kStageCap) {
+			// The block does not fit: flag it and release the task untouched.
+			if (lane == 0) {
+				atomicOr(T.error, kErrStageOverflow);
+				st_release(&T.done[t], 1u);
+			}
+			__syncwarp();
+			continue;
+		}
+		if (L > C::kVelCap) {
+			slot_far_task<C>(S, s, L, first, cnt, sc.p, P.vel, P.pos, lane);
+		} else {
+			slot_copy_vel<C>(S, s, L, segStart, segOff, P, lane, true);
+			stamp(T, 0, t, 2, lane);
+			float2 xi = __ldg(&P.pos[first]);
+			for (int k = 0; k < cnt; ++k) {
+				const float2 xn = __ldg(&P.pos[first + min(k + 1, cnt - 1)]);
+				seg.own = 8 * (own + k) + kSegFirst;
+				bool listed = false;
+				if (regs) {
+					// One segment: all of the particle's pairs, if they fit.
+					float4 *G = S.slot[s].geo[seg.seq & 1u];
+					int m = 0;
+#pragma unroll
+					for (int r = 0; r < C::kRegEntries; ++r) {
+						if (r * kWarp >= L) break;
+						const float rx = px[r].x - xi.x, ry = px[r].y - xi.y;
+						const float r2 = rx * rx + ry * ry;
+						const bool in = r2 < h2;
+						const unsigned mask = __ballot_sync(kFull, in);
+						const int at = m + __popc(mask & lanemask_lt());
+						if (in && at < C::kGeom) G[at] = make_float4(__int_as_float(8 * (r * kWarp + lane)), rx, ry, r2);
+						m += __popc(mask);
+					}
+					listed = m <= C::kGeom;
+					if (listed) seg.m = m;
+				}
+				if (!listed) {
+					for (int b0 = 0; b0 < L; b0 += kWarp) {
+						const int e = b0 + lane;
+						const float2 xj = e < L ? __ldg(&P.pos[seg_src<9>(e, segOff, segStart)]) : xi;
+						if (!slot_entries<C>(S, s, seg, 8 * e, xj, e < L, xi, h2, invH, sc.p, T, lane)) return;
+					}
+				}
+				if (!slot_publish<C>(S, s, seg, true, invH, sc.p, T, lane)) return;
+				xi = xn;
+			}
+			if (!slot_taken<C>(S, s, seg.seq, T)) return;
+			slot_copy_vel<C>(S, s, L, segStart, segOff, P, lane, false);
+		}
+		__threadfence();
+		__syncwarp();
+		stamp(T, 0, t, 3, lane);
+		if (lane == 0 && i != T.hold[0]) st_release(&T.done[t], 1u);
 	}
-	const int len = m > C::kGeom ? 0 : m;
-	visc_chain(V, S.slot[s].geo[buf], &S.idle, len, __reduce_max_sync(running, len), vi, sigma, beta, hdt);
-	V[own] = vi;
 }
 
 }  // namespace
 
 template <class C>
-__global__ void __launch_bounds__(C::kWarps * kWarp, C::kMinBlocks) k_viscosity_multi(Totals tt, Particles P,
-                                                                                     SimTables T) {
+__global__ void __launch_bounds__(C::kThreads, C::kMinBlocks) k_viscosity_multi(Totals tt, Particles P,
+                                                                                           SimTables T) {
 	extern __shared__ __align__(16) unsigned char smem_raw[];
 	ViscMultiSmemT<C> &S = *reinterpret_cast<ViscMultiSmemT<C> *>(smem_raw);
 	const int tid = threadIdx.x, warp = tid / kWarp, lane = tid & (kWarp - 1);
-	const int nLive = *T.nLive;
 	if (tid < C::kSlots) {
-		S.state[tid] = kSlotFree;
-		S.k[tid] = 0;
+		S.ready[tid] = 0;
+		S.taken[tid] = 0;
 	}
 	if (tid == 0) {
-		S.exhausted = 0;
-		S.aborted = 0;
+		S.exited = 0;
 		S.idle = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
 	}
 	__syncthreads();
-	for (;;) {
-		// Bookkeeping of the phase just ended: thread s advances slot s.
-		int busy = 0;
-		if (tid < C::kSlots) {
-			int st = S.state[tid];
-			if (st == kSlotStaged) {
-				st = kSlotRun;
-				S.k[tid] = 0;
-			} else if (st == kSlotRun) {
-				const int k = S.k[tid] + 1;
-				S.k[tid] = k;
-				if (k == S.cnt[tid]) st = kSlotDone;
-			}
-			S.state[tid] = st;
-			busy = st != kSlotFree;
-		}
-		const int anyBusy = __syncthreads_or(busy);
-		if ((!anyBusy && S.exhausted) || S.aborted) break;
-		if (warp == 0) {
-			const bool run = lane < C::kSlots && S.state[lane] == kSlotRun;
-			const unsigned running = __ballot_sync(kFull, run);
-			if (run) slot_chain<C>(S, lane, running, P);
-		} else {
-			if (tid == kWarp && ld_acquire(T.abort) != 0u) S.aborted = 1;
-			__syncwarp();
-			for (int s = warp - 1; s < C::kSlots; s += C::kProd) slot_produce<C>(S, s, P, T, nLive, lane);
-		}
-		__syncthreads();
+	if (warp < C::kChains) {
+		slot_chains<C>(S, warp * (C::kSlots / C::kChains), lane);
+	} else {
+		slot_producer<C>(S, warp - C::kChains, P, T, *T.nLive, lane);
+		__syncwarp();
+		if (lane == 0) atomicAdd(&S.exited, 1);
 	}
 }
 
@@ -2600,7 +2749,7 @@ cudaError_t sweep_attributes() {
 
 cudaError_t sweep_occupancy(bool viscLean, int deltaShape, int *occV, int *occD) {
 	cudaError_t e = viscLean ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(occV, k_viscosity_multi<ViscLean>,
-	                                                                         ViscLean::kWarps * kWarp,
+	                                                                         ViscLean::kThreads,
 	                                                                         sizeof(ViscMultiSmemT<ViscLean>))
 	                         : cudaOccupancyMaxActiveBlocksPerMultiprocessor(occV, k_viscosity<ViscWide>,
 	                                                                         ViscWide::kWarps * kWarp,
@@ -2628,7 +2777,7 @@ cudaError_t sweep_occupancy(bool viscLean, int deltaShape, int *occV, int *occD)
 void launch_viscosity(bool lean, int blocks, cudaStream_t st, Totals tt, Particles P, SimTables T) {
 	if (lean)
 		k_viscosity_multi<ViscLean>
-		    <<<blocks, ViscLean::kWarps * kWarp, sizeof(ViscMultiSmemT<ViscLean>), st>>>(tt, P, T);
+		    <<<blocks, ViscLean::kThreads, sizeof(ViscMultiSmemT<ViscLean>), st>>>(tt, P, T);
 	else
 		k_viscosity<ViscWide><<<blocks, ViscWide::kWarps * kWarp, visc_smem_bytes<ViscWide>(), st>>>(tt, P, T);
 }

@@ -12,10 +12,16 @@ namespace sphgb {
 struct ViscWide {
 	static constexpr int kWarps = 4, kProducers = 3 * kWarp, kGeom = 512, kMinBlocks = 4;
 };
-// Lean viscosity: kSlots tasks per block; warp 0's lanes run their chains,
-// kProd producer warps serve them (k_viscosity_multi).
+// Lean viscosity: kSlots tasks per block, one block per SM; the lanes of
+// kChains warps run their chains, one producer warp serves each
+// (k_viscosity_multi).  A slot stages up to kVelCap list entries; its producer
+// holds the positions of up to kRegEntries * 32 of them in registers.  kName:
+// the number that names the shape in sph_set_sweep_shape.
 struct ViscLean {
-	static constexpr int kSlots = 5, kProd = 4, kWarps = 1 + kProd, kGeom = 192, kMinBlocks = 3;
+	static constexpr int kName = 5;
+	static constexpr int kSlots = 18, kChains = 2, kVelCap = 768, kGeom = 160, kRegEntries = 12, kMinBlocks = 1;
+	static constexpr int kThreads = (kChains + kSlots) * kWarp;
+	static_assert(kSlots % kChains == 0 && kSlots / kChains <= kWarp && kGeom >= kWarp, "slots per chain warp");
 };
 // Delta sweep.  Pipelined shapes run kWarps - 1 producer warps and one
 // summer warp per task; the others relax one particle at a time on the
