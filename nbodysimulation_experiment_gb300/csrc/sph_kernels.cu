@@ -36,6 +36,7 @@
 // order, so per-pair results are bit-identical to the reference.
 #include "sph_internal.cuh"
 #include "sph_kernels.cuh"
+#include "sph_math.cuh"
 
 namespace sphgb {
 
@@ -102,17 +103,6 @@ __device__ __forceinline__ int cell_of(float2 p, const StepParams &s) {
 	x = min(max(x, 0), s.gx - 1);
 	y = min(max(y, 0), s.gy - 1);
 	return y * s.gx + x;
-}
-
-// r = sqrt(r2) and 1 / r, or r = 0 and 1 for coinciding points (Vec2Normalize
-// keeps a zero vector).  Every particle meets itself in its own list, and the
-// root of 0 would send its warp down the slow path of sqrtf each time; the
-// root of 1 gives the same two results.
-__device__ __forceinline__ float root_and_inverse(float r2, float &r) {
-	const bool zero = r2 == 0.0f;
-	const float len = sqrtf(zero ? 1.0f : r2);
-	r = zero ? 0.0f : len;
-	return 1.0f / len;
 }
 
 __device__ __forceinline__ int rect_dist(int ax0, int ay0, int ax1, int ay1, int bx0, int by0, int bx1, int by1) {
@@ -427,11 +417,9 @@ __device__ __forceinline__ void visc_wave(ViscSmemT<C> &S, int k, int cnt, int o
 			const float rx = xj.x - xi.x, ry = xj.y - xi.y;
 			const float r2 = rx * rx + ry * ry;
 			if (!(r2 < s.h2)) continue;
-			const float r = sqrtf(r2);
+			float r;
+			const float inv = root_and_inverse(r2, r);
 			const float qq = r * s.invH;
-			float lenr = r;
-			if (lenr == 0.0f) lenr = 1.0f;
-			const float inv = 1.0f / lenr;
 			visc_pair(base + 8u * e, make_float2(rx * inv, ry * inv), 1.0f - qq, S.vel[e], vi, s.sigma, s.beta, hdt);
 		}
 		return;
@@ -1903,11 +1891,11 @@ __device__ __forceinline__ float2 delta_half(float2 xj, float2 xk, float r2, flo
 // component each.  In isolation 112 pairs take 685 cycles, 818 in batches of
 // eight; one lane subtracting both components took 9.4 cycles a pair.
 __device__ __forceinline__ float sum_halves(const float *H, int n, float dx) {
-	const float4 *H4 = reinterpret_cast<const float4 *>(H);
+	const uint32_t h = shared_addr(H);
 	for (int b = 0; b < n; b += kSumPad) {
 		float4 a[kSumPad / 4];
 #pragma unroll
-		for (int u = 0; u < kSumPad / 4; ++u) a[u] = H4[b / 4 + u];
+		for (int u = 0; u < kSumPad / 4; ++u) a[u] = lds4(h + 4u * b + 16u * u);
 #pragma unroll
 		for (int u = 0; u < kSumPad / 4; ++u) dx = dx - a[u].x - a[u].y - a[u].z - a[u].w;
 	}
@@ -2258,6 +2246,10 @@ __device__ __forceinline__ unsigned long long relax_group(DeltaSmemT<C> &S, int 
 								for (int i = 1; i < kE; ++i) at[i] = direct_slot<C>(sl, ln, tid, i);
 								if (ln.w <= 2 * kWarp)
 									produce_direct<C, 2>(S, b, at, sl.w, pk, pend, below, s, tid);
+								else if (kE > 4 && ln.w <= 4 * kWarp)
+									produce_direct<C, (kE > 4 ? 4 : kE)>(S, b, at, sl.w, pk, pend, below, s, tid);
+								else if (kE > 6 && ln.w <= 6 * kWarp)
+									produce_direct<C, (kE > 6 ? 6 : kE)>(S, b, at, sl.w, pk, pend, below, s, tid);
 								else
 									produce_direct<C, kE>(S, b, at, sl.w, pk, pend, below, s, tid);
 							}
