@@ -1689,7 +1689,7 @@ __global__ void __launch_bounds__(kDensWarps * kWarp, 4) k_density(Totals tt, Pa
 // slot) are worked out for a chunk of particles at once, off the serial path.
 //
 // Particles are relaxed in a two-stage pipeline.  In phase k the producer
-// warps (all but the last) scan particle k's list, compact the in-range pairs
+// warps scan particle k's list, compact the in-range pairs
 // in list order and evaluate them (x_j += D/2), while the summer warp (the
 // last) finishes particle k-1: its ordered sum dx -= D/2 and x_{k-1} += dx.
 // The only pair of particle k that needs x_{k-1} after that sum is
@@ -1702,14 +1702,11 @@ __global__ void __launch_bounds__(kDensWarps * kWarp, 4) k_density(Totals tt, Pa
 // before reading it.
 // Particles whose lists exceed one pass, and regions staged particle by
 // particle, drain the pipeline and run on the whole block in turn.
-// Three shapes (sph_kernels.cuh): wide is pipelined with eleven producer
-// warps, one block per SM (short per-particle latency, one scene); mid is
-// pipelined with seven, two blocks per SM; lean is two warps without the
-// pipeline and with smaller staging (more tasks per SM, many scenes).
+// The shapes and what each is for: sph_kernels.cuh.
 constexpr int kSumPad = 32;  // +0 entries past the last half, at most one batch of the sum
 template <class C>
 struct DeltaSmemT {
-	static constexpr int kProd = C::kWarps - 1;         // producer warps
+	static constexpr int kProd = C::kProducers;         // producer warps
 	static constexpr int kPass = kProd * C::kChainW;    // list entries per pipelined particle
 	static constexpr int kSeqPass = C::kWarps * C::kChainW;  // list entries per pass, whole block
 	static constexpr int kHalf = (kSeqPass > kPass ? kSeqPass : kPass) + 36;  // 4 past a multiple of the 32 banks
@@ -1883,6 +1880,24 @@ __device__ __forceinline__ float2 delta_half(float2 xj, float2 xk, float r2, flo
 	return make_float2(d * nx * 0.5f, d * ny * 0.5f);
 }
 
+// The same without a branch, for r2 = 0 or in the plain range of root_plain;
+// and for any distance, out of line.
+__device__ __forceinline__ float2 delta_half_line(float2 xj, float2 xk, float r2, float2 pk, const StepParams &s) {
+	const float rx = xj.x - xk.x, ry = xj.y - xk.y;
+	const bool zero = r2 == 0.0f;
+	float len;
+	const float inv = inverse_root_line(zero ? 1.0f : r2, len);
+	const float rij = zero ? 0.0f : len;
+	const float nx = rx * inv, ny = ry * inv;
+	const float term = 1.0f - rij * s.invH;
+	const float d = s.dt2 * (pk.x * term + pk.y * (term * term));
+	return make_float2(d * nx * 0.5f, d * ny * 0.5f);
+}
+__device__ __noinline__ float2 delta_half_any(float2 xj, float2 xk, float2 pk, const StepParams &s) {
+	const float rx = xj.x - xk.x, ry = xj.y - xk.y;
+	return delta_half(xj, xk, rx * rx + ry * ry, pk, s);
+}
+
 // dx -= delta * 0.5 over the n buffered halves of one component, in list
 // order (demo4.cpp:251), starting at dx: one dependent subtraction per pair
 // (four cycles), in batches of 32 loaded at once, so that a batch's loads and
@@ -2008,9 +2023,9 @@ __device__ __forceinline__ void producers_bar() {
 // pair with slot `prev` (the particle still being finished, or -1).
 template <class C>
 __device__ __forceinline__ void produce(DeltaSmemT<C> &S, int b, int4 sl, int4 ln, float2 pk, int prev,
-                                        const StepParams &s, int tid) {
+                                        const StepParams &s, int warp, int lane) {
 	constexpr int kP = DeltaSmemT<C>::kProd;
-	const int lane = tid & (kWarp - 1), warp = tid / kWarp;
+	const int tid = warp * kWarp + lane;
 	const int own = sl.w;
 	const int len0 = ln.x, l01 = ln.x + ln.y, L = l01 + ln.z;
 	const float2 xk = S.pos[own];
@@ -2062,16 +2077,16 @@ __device__ __forceinline__ void produce(DeltaSmemT<C> &S, int b, int4 sl, int4 l
 // per particle, 2,060 when every warp compacted first.
 template <class C, int R>
 __device__ __forceinline__ void produce_direct(DeltaSmemT<C> &S, int b, const int *at, int own, float2 pk, int prev,
-                                               uint4 below, const StepParams &s, int tid) {
+                                               uint4 below, const StepParams &s, int warp, int lane) {
 	constexpr int kP = DeltaSmemT<C>::kProd;
 	static_assert(kP <= 16 && C::kChainW < 256, "a phase's counts are one 16-byte word");
-	const int lane = tid & (kWarp - 1), warp = tid / kWarp;
 	const float2 xk = S.pos[own];
 	float2 xj[R], h[R];
 	unsigned mask[R];
 	bool in[R];
 	int cnt = 0;
-	if (tid == 0) S.meta[b] = make_int4(0, -1, own, 0);
+	bool plain = true;
+	if (warp == 0 && lane == 0) S.meta[b] = make_int4(0, -1, own, 0);
 #pragma unroll
 	for (int i = 0; i < R; ++i) xj[i] = S.pos[max(at[i], 0)];
 #pragma unroll
@@ -2083,7 +2098,12 @@ __device__ __forceinline__ void produce_direct(DeltaSmemT<C> &S, int b, const in
 		in[i] = at[i] >= 0 && at[i] != prev && r2 < s.h2;
 		mask[i] = __ballot_sync(kFull, in[i] || (at[i] >= 0 && at[i] == prev));
 		cnt += __popc(mask[i]);
-		h[i] = delta_half(xj[i], xk, r2, pk, s);
+		h[i] = delta_half_line(xj[i], xk, r2, pk, s);
+		plain = plain && (!in[i] || r2 == 0.0f || root_plain(r2));
+	}
+	if (!plain) {
+#pragma unroll
+		for (int i = 0; i < R; ++i) h[i] = delta_half_any(xj[i], xk, pk, s);
 	}
 	if (lane == 0) S.wcnt8[warp] = (unsigned char)cnt;
 #pragma unroll
@@ -2126,19 +2146,20 @@ __device__ __forceinline__ uint4 warps_below(int warp) {
 	return make_uint4(m[0], m[1], m[2], m[3]);
 }
 
-// The list entry of this producer thread in round i (a staged slot, or -1) for
-// the particle with row ranges sl, ln.
+// The list entry of lane `lane` of producer warp `warp` in round i (a staged
+// slot, or -1) for the particle with row ranges sl, ln.
 template <class C>
-__device__ __forceinline__ int direct_slot(int4 sl, int4 ln, int tid, int i) {
-	const int r = i * kWarp + (tid & (kWarp - 1));
-	const int e = (tid / kWarp) * ln.w + r;
+__device__ __forceinline__ int direct_slot(int4 sl, int4 ln, int warp, int lane, int i) {
+	const int r = i * kWarp + lane;
+	const int e = warp * ln.w + r;
 	const int l01 = ln.x + ln.y;
 	// Rows start at sl.x, sl.y - ln.x and sl.z - l01 of the flat list.
 	const int base = e < ln.x ? sl.x : (e < l01 ? sl.y - ln.x : sl.z - l01);
 	return r < ln.w && e < l01 + ln.z ? base + e : -1;
 }
 
-// Summer's part of a phase (lanes c = 0 and 1 of the warp: x and y): finish
+// Summer's part of a phase (a whole warp: even lanes take the x component,
+// odd lanes the y, all of them the same way, so that nothing diverges): finish
 // the previous particle `prev` (buffer b ^ 1), then evaluate the pair (k, k-1)
 // of particle k (list slots sl, ln, pressures pk) if k-1 is in k's list; this
 // component of its D/2 goes to hres.  What does not depend on the sum is
@@ -2150,7 +2171,7 @@ __device__ __forceinline__ void summer(DeltaSmemT<C> &S, int b, int c, int prev,
 	const bool inList = (prev >= sl.x && prev < sl.x + ln.x) || (prev >= sl.y && prev < sl.y + ln.y) ||
 	                    (prev >= sl.z && prev < sl.z + ln.z);
 	float x = finish_sum<C>(S, b ^ 1, c, hres);
-	const float o = __shfl_xor_sync(0x3u, x, 1);
+	const float o = __shfl_xor_sync(kFull, x, 1);
 	const float2 xp = c == 0 ? make_float2(x, o) : make_float2(o, x);
 	const float rx = xp.x - xk.x, ry = xp.y - xk.y;
 	const float r2 = rx * rx + ry * ry;
@@ -2158,6 +2179,92 @@ __device__ __forceinline__ void summer(DeltaSmemT<C> &S, int b, int c, int prev,
 	const bool in = inList && r2 < s.h2;
 	hres = in ? h : 0.0f;
 	*comp_of(&S.pos[prev], c) = in ? h + x : x;
+}
+
+// Role of a warp in the pipeline: a producer's number, kProd for the summer,
+// or -1 (kApart: the summer is warp 3 and the other warps of its scheduler
+// stay out, so that no producer takes its issue slots).  The summer's dependent
+// subtractions lose a cycle whenever another warp issues in their place:
+// one task of 36 particles alone, wide shape, 799 ns per particle with three
+// warps on each scheduler and both roles in one loop, 636 apart in loops of
+// their own (dense 857 -> 637, quad 1,216 -> 1,148).
+template <class C>
+__device__ __forceinline__ int pipeline_role(int warp) {
+	if (!C::kApart) return warp;
+	return (warp & 3) != 3 ? (warp >> 2) * 3 + (warp & 3) : (warp == 3 ? DeltaSmemT<C>::kProd : -1);
+}
+template <class C>
+__device__ __forceinline__ bool pipelinable(int4 sl, int4 ln) {
+	return C::kPipelined && sl.w >= 0 && ln.x + ln.y + ln.z <= DeltaSmemT<C>::kPass;
+}
+template <class C>
+__device__ __forceinline__ void phase_bar() {
+	__syncwarp();
+	asm volatile("bar.sync 2, %0;" ::"r"((DeltaSmemT<C>::kProd + 1) * kWarp) : "memory");
+}
+
+// One particle on the producers.
+template <class C>
+__device__ __forceinline__ void produce_phase(DeltaSmemT<C> &S, int b, int4 sl, int4 ln, float2 pk, int at0, int prev,
+                                              uint4 below, const StepParams &s, int role, int lane) {
+	if constexpr (C::kDirect) {
+		constexpr int kE = C::kChainW / kWarp;
+		if (ln.w <= kWarp) {
+			produce_direct<C, 1>(S, b, &at0, sl.w, pk, prev, below, s, role, lane);
+			return;
+		}
+		int at[kE];
+		at[0] = at0;
+#pragma unroll
+		for (int i = 1; i < kE; ++i) at[i] = direct_slot<C>(sl, ln, role, lane, i);
+		if (ln.w <= 2 * kWarp)
+			produce_direct<C, 2>(S, b, at, sl.w, pk, prev, below, s, role, lane);
+		else if (kE > 4 && ln.w <= 4 * kWarp)
+			produce_direct<C, (kE > 4 ? 4 : kE)>(S, b, at, sl.w, pk, prev, below, s, role, lane);
+		else
+			produce_direct<C, kE>(S, b, at, sl.w, pk, prev, below, s, role, lane);
+	} else {
+		produce<C>(S, b, sl, ln, pk, prev, s, role, lane);
+	}
+}
+
+// The pipelined particles from index i on of the chunk's n: each role loops on
+// its own, meeting the others at the end of every phase, until the chunk ends
+// or a particle has to run on the whole block.  Returns that index; `ph` counts
+// phases and `prev` is the pending particle's slot (-1: none).
+template <class C>
+__device__ __forceinline__ int run_pipeline(DeltaSmemT<C> &S, int i, int n, int &ph, int &prev, float &hres, uint4 below,
+                                            const StepParams &s, int role, int lane) {
+	constexpr int kP = DeltaSmemT<C>::kProd;
+	int4 sl = S.pslot[i], ln = S.plen[i];
+	if (role < 0) {
+		for (; i < n; ++i, ++ph) {
+			const int4 a = S.pslot[i], l = S.plen[i];
+			if (!pipelinable<C>(a, l)) break;
+			prev = a.w;
+		}
+		return i;
+	}
+	float2 pk = S.ppk[i];
+	int at0 = role < kP && C::kDirect ? direct_slot<C>(sl, ln, role, lane, 0) : 0;
+	for (;;) {
+		const int next = min(i + 1, n - 1), b = (ph & 1) % DeltaSmemT<C>::kPhases;
+		const int4 slN = S.pslot[next], lnN = S.plen[next];
+		const float2 pkN = S.ppk[next];
+		if (role < kP) {
+			produce_phase<C>(S, b, sl, ln, pk, at0, prev, below, s, role, lane);
+			if (C::kDirect) at0 = direct_slot<C>(slN, lnN, role, lane, 0);
+		} else if (prev >= 0) {
+			summer<C>(S, b, lane & 1, prev, sl, ln, pk, s, hres);
+		}
+		phase_bar<C>();
+		prev = sl.w;
+		++ph;
+		if (++i >= n || !pipelinable<C>(slN, lnN)) return i;
+		sl = slN;
+		ln = lnN;
+		pk = pkN;
+	}
 }
 
 // Process particles [p0, p1) (old numbers, or positions in AddParticle order
@@ -2193,10 +2300,10 @@ __device__ __forceinline__ unsigned long long relax_group(DeltaSmemT<C> &S, int 
 	}
 	const bool staged = stage_region<C>(S, R, Q, T, s, cellBase, tid);
 	const unsigned long long tStaged = global_ns();
-	bool pending = false;  // the previous particle still needs its sum (buffer ph ^ 1)
-	int ph = 0, prev = -1;  // prev: the pending particle's slot
-	float hres = 0.0f;  // summer lanes: this component of D/2 of the pending particle's reserved pair
-	const uint4 below = warps_below(warp);
+	int ph = 0, prev = -1;  // prev: slot of the particle whose sum is pending (buffer ph ^ 1), or -1
+	float hres = 0.0f;      // summer: this component of D/2 of the pending particle's reserved pair
+	const int role = pipeline_role<C>(warp);
+	const uint4 below = warps_below(max(role, 0));
 	for (int c0 = p0; c0 < p1; c0 += C::kPrefetch) {
 		const int c1 = min(p1, c0 + C::kPrefetch);
 		for (int k = c0 + tid; k < c1; k += kDT) {
@@ -2213,66 +2320,21 @@ __device__ __forceinline__ unsigned long long relax_group(DeltaSmemT<C> &S, int 
 			}
 		}
 		__syncthreads();
-		// A particle's inputs are loaded a phase ahead (kDirect: this thread's
-		// first list entry too), beside the arithmetic of the current one.
-		int4 slN = make_int4(0, 0, 0, -1), lnN = make_int4(0, 0, 0, 0);
-		float2 pkN = S.ppk[0];
-		int atN = -1;
-		if (staged) {
-			slN = S.pslot[0];
-			lnN = S.plen[0];
-			if (C::kDirect && warp < kP) atN = direct_slot<C>(slN, lnN, tid, 0);
-		}
-		for (int k = c0; k < c1; ++k) {
+		for (int k = c0; k < c1;) {
 			if (staged) {
-				const int4 sl = slN, ln = lnN;
-				const float2 pk = pkN;
-				const int at0 = atN, kn = min(k + 1, c1 - 1) - c0;
-				slN = S.pslot[kn];
-				lnN = S.plen[kn];
-				pkN = S.ppk[kn];
-				if (C::kPipelined && sl.w >= 0 && ln.x + ln.y + ln.z <= DeltaSmemT<C>::kPass) {
-					const int b = (ph & 1) % DeltaSmemT<C>::kPhases;
-					const int pend = pending ? prev : -1;
-					if (warp < kP) {
-						if constexpr (C::kDirect) {
-							constexpr int kE = C::kChainW / kWarp;
-							if (ln.w <= kWarp) {
-								produce_direct<C, 1>(S, b, &at0, sl.w, pk, pend, below, s, tid);
-							} else {
-								int at[kE];
-								at[0] = at0;
-#pragma unroll
-								for (int i = 1; i < kE; ++i) at[i] = direct_slot<C>(sl, ln, tid, i);
-								if (ln.w <= 2 * kWarp)
-									produce_direct<C, 2>(S, b, at, sl.w, pk, pend, below, s, tid);
-								else if (kE > 4 && ln.w <= 4 * kWarp)
-									produce_direct<C, (kE > 4 ? 4 : kE)>(S, b, at, sl.w, pk, pend, below, s, tid);
-								else if (kE > 6 && ln.w <= 6 * kWarp)
-									produce_direct<C, (kE > 6 ? 6 : kE)>(S, b, at, sl.w, pk, pend, below, s, tid);
-								else
-									produce_direct<C, kE>(S, b, at, sl.w, pk, pend, below, s, tid);
-							}
-							atN = direct_slot<C>(slN, lnN, tid, 0);
-						} else {
-							produce<C>(S, b, sl, ln, pk, pend, s, tid);
-						}
-					} else if (pending && lane < 2) {
-						summer<C>(S, b, lane, prev, sl, ln, pk, s, hres);
-					}
+				const int4 sl = S.pslot[k - c0], ln = S.plen[k - c0];
+				if (pipelinable<C>(sl, ln)) {
+					k = c0 + run_pipeline<C>(S, k - c0, c1 - c0, ph, prev, hres, below, s, role, lane);
 					__syncthreads();
-					prev = sl.w;
-					pending = true;
-					++ph;
 					continue;
 				}
-				if (C::kDirect && warp < kP) atN = direct_slot<C>(slN, lnN, tid, 0);
 				// Drain the pipeline, then relax this particle on the whole block.
-				if (C::kPipelined && pending && warp == kP && lane < 2)
-					*comp_of(&S.pos[prev], lane) = finish_sum<C>(S, (ph & 1) ^ 1, lane, hres);
+				if (C::kPipelined && prev >= 0 && role == kP)
+					*comp_of(&S.pos[prev], lane & 1) = finish_sum<C>(S, (ph & 1) ^ 1, lane & 1, hres);
 				__syncthreads();
-				pending = false;
-				relax_particle<C>(S, sl, ln, pk, s, tid);
+				prev = -1;
+				relax_particle<C>(S, sl, ln, S.ppk[k - c0], s, tid);
+				++k;
 				continue;
 			}
 			const int nc = S.pnc[k - c0], jk = S.pjk[k - c0];
@@ -2286,6 +2348,7 @@ __device__ __forceinline__ unsigned long long relax_group(DeltaSmemT<C> &S, int 
 			if (!stage_region<C>(S, R1, Q, T, s, cellBase, tid)) {
 				if (tid == 0) atomicOr(T.error, kErrStageOverflow);
 				__syncthreads();
+				++k;
 				continue;
 			}
 			if (tid == 0) particle_slots<C>(S, R1, nc, jk, s, cellBase, T.error, S.oneSlot, S.oneLen);
@@ -2293,11 +2356,12 @@ __device__ __forceinline__ unsigned long long relax_group(DeltaSmemT<C> &S, int 
 			relax_particle<C>(S, S.oneSlot, S.oneLen, pk, s, tid);
 			write_back_owned<C>(S, R1, Q, tid);
 			__syncthreads();
+			++k;
 		}
 		__syncthreads();
 	}
-	if (C::kPipelined && pending && warp == kP && lane < 2)
-		*comp_of(&S.pos[prev], lane) = finish_sum<C>(S, (ph & 1) ^ 1, lane, hres);
+	if (C::kPipelined && prev >= 0 && role == kP)
+		*comp_of(&S.pos[prev], lane & 1) = finish_sum<C>(S, (ph & 1) ^ 1, lane & 1, hres);
 	__syncthreads();
 	if (staged) write_back_owned<C>(S, R, Q, tid);
 	return tStaged;
