@@ -1703,6 +1703,11 @@ __global__ void __launch_bounds__(kDensWarps * kWarp, 4) k_density(Totals tt, Pa
 // Particles whose lists exceed one pass, and regions staged particle by
 // particle, drain the pipeline and run on the whole block in turn.
 // The shapes and what each is for: sph_kernels.cuh.
+// Rounds of 32 list entries a scanning warp loads at once (tri, quad, lean).
+// One task of 36 particles alone, ns per particle, one round at a time and
+// evaluated after the other warps' counts: 1,445, 1,148, 1,700; two at once
+// 1,343, 1,080, 1,568; four 1,316, 1,046, 1,566; six 1,273, 1,086, 1,524.
+constexpr int kScanBatch = 4;
 constexpr int kSumPad = 32;  // +0 entries past the last half, at most one batch of the sum
 template <class C>
 struct DeltaSmemT {
@@ -1929,29 +1934,36 @@ __device__ __forceinline__ int scan_range(float4 *cand, int nw, int w, int lane,
                                           float2 *ownAfter) {
 	const int per = (pl + nw - 1) / nw;
 	const int e0 = p0 + w * per, e1 = min(p0 + pl, e0 + per);
+	// Rows start at sl.x, sl.y - len0 and sl.z - l01 of the flat list.
+	const int row1 = sl.y - len0, row2 = sl.z - l01;
 	int cnt = 0;
-	for (int eb = e0; eb < e1; eb += kWarp) {
-		const int e = eb + lane;
-		bool in = false;
-		int slot = 0;
-		float2 xj = make_float2(0.f, 0.f);
-		float r2 = 0.f;
-		if (e < e1) {
-			slot = e < len0 ? sl.x + e : (e < l01 ? sl.y + (e - len0) : sl.z + (e - l01));
-			if (slot == skip) {
-				in = true;
-				r2 = -1.0f;
-			} else {
-				xj = pos[slot];
-				const float rx = xj.x - xk.x, ry = xj.y - xk.y;
-				r2 = rx * rx + ry * ry;
-				in = r2 < h2;
-				if (slot == own) *ownAfter = xj;  // out of range: no displacement
-			}
+	for (int eb = e0; eb < e1; eb += kScanBatch * kWarp) {
+		float2 xj[kScanBatch];
+		int slot[kScanBatch];
+#pragma unroll
+		for (int u = 0; u < kScanBatch; ++u) {
+			const int e = eb + u * kWarp + lane;
+			slot[u] = e < e1 ? e + (e < len0 ? sl.x : (e < l01 ? row1 : row2)) : -1;
+			xj[u] = pos[max(slot[u], 0)];
 		}
-		const unsigned mk = __ballot_sync(kFull, in);
-		if (in) cand[cnt + __popc(mk & lanemask_lt())] = make_float4(__int_as_float(slot), xj.x, xj.y, r2);
-		cnt += __popc(mk);
+#pragma unroll
+		for (int u = 0; u < kScanBatch; ++u) {
+			if (eb + u * kWarp >= e1) break;
+			const float rx = xj[u].x - xk.x, ry = xj[u].y - xk.y;
+			float r2 = rx * rx + ry * ry;
+			bool in = slot[u] >= 0 && r2 < h2;
+			if (slot[u] >= 0) {
+				if (slot[u] == skip) {
+					in = true;
+					r2 = -1.0f;
+				} else if (slot[u] == own) {
+					*ownAfter = xj[u];  // out of range: no displacement
+				}
+			}
+			const unsigned mk = __ballot_sync(kFull, in);
+			if (in) cand[cnt + __popc(mk & lanemask_lt())] = make_float4(__int_as_float(slot[u]), xj[u].x, xj[u].y, r2);
+			cnt += __popc(mk);
+		}
 	}
 	return cnt;
 }
@@ -2024,17 +2036,49 @@ __device__ __forceinline__ void producers_bar() {
 template <class C>
 __device__ __forceinline__ void produce(DeltaSmemT<C> &S, int b, int4 sl, int4 ln, float2 pk, int prev,
                                         const StepParams &s, int warp, int lane) {
-	constexpr int kP = DeltaSmemT<C>::kProd;
-	const int tid = warp * kWarp + lane;
+	constexpr int kP = DeltaSmemT<C>::kProd, R = 2;
 	const int own = sl.w;
 	const int len0 = ln.x, l01 = ln.x + ln.y, L = l01 + ln.z;
 	const float2 xk = S.pos[own];
-	if (tid == 0) S.meta[b].y = -1;
+	if (warp == 0 && lane == 0) S.meta[b] = make_int4(0, -1, own, 0);
+	const float4 *cand = S.cand[warp];
 	const int cnt = scan_range(S.cand[warp], kP, warp, lane, 0, L, sl, len0, l01, xk, own, prev, S.pos, s.h2,
 	                           &S.ownAfter[b]);
+	if (lane == 0) S.wcnt[warp] = cnt;
+	__syncwarp();
+	// The candidates of the first R rounds side by side, before the counts of
+	// the other warps are needed; what is left after that, one by one.
+	auto apply = [&](float4 cd, float2 h) {
+		const int slot = __float_as_int(cd.x);
+		const float2 moved = make_float2(h.x + cd.y, h.y + cd.z);
+		if (slot == own) S.ownAfter[b] = moved; else S.pos[slot] = moved;
+	};
+	auto place = [&](float4 cd, float2 h, int at) {
+		if (cd.w < 0.0f) {
+			S.meta[b].y = at;  // (k, k-1): the summer evaluates it
+		} else {
+			S.half[b][0][at] = h.x;
+			S.half[b][1][at] = h.y;
+		}
+	};
+	float4 cd[R];
+	float2 h[R];
+	bool plain = true;
+#pragma unroll
+	for (int i = 0; i < R; ++i) {
+		cd[i] = cand[min(i * kWarp + lane, C::kChainW - 1)];
+		h[i] = delta_half_line(make_float2(cd[i].y, cd[i].z), xk, cd[i].w, pk, s);
+		plain = plain && (i * kWarp + lane >= cnt || cd[i].w <= 0.0f || root_plain(cd[i].w));
+	}
+	if (!plain) {
+#pragma unroll
+		for (int i = 0; i < R; ++i) h[i] = delta_half_any(make_float2(cd[i].y, cd[i].z), xk, pk, s);
+	}
+#pragma unroll
+	for (int i = 0; i < R; ++i)
+		if (i * kWarp + lane < cnt && cd[i].w >= 0.0f) apply(cd[i], h[i]);
 	int before = 0, total = cnt;
 	if (kP > 1) {
-		if (lane == 0) S.wcnt[warp] = cnt;
 		producers_bar<C>();
 		total = 0;
 #pragma unroll
@@ -2043,27 +2087,19 @@ __device__ __forceinline__ void produce(DeltaSmemT<C> &S, int b, int4 sl, int4 l
 			before += (w < warp) ? c : 0;
 			total += c;
 		}
-	} else {
-		__syncwarp();
 	}
-	if (tid < kSumPad) S.half[b][0][total + tid] = S.half[b][1][total + tid] = 0.0f;
-	for (int q = lane; q < cnt; q += kWarp) {
-		const float4 cd = S.cand[warp][q];
-		if (cd.w < 0.0f) {
-			S.meta[b].y = before + q;  // (k, k-1): the summer evaluates it
-			continue;
-		}
-		const float2 xj = make_float2(cd.y, cd.z);
-		const float2 h = delta_half(xj, xk, cd.w, pk, s);
-		const int slot = __float_as_int(cd.x);
-		const float2 moved = make_float2(h.x + xj.x, h.y + xj.y);
-		if (slot == own) S.ownAfter[b] = moved; else S.pos[slot] = moved;
-		S.half[b][0][before + q] = h.x;
-		S.half[b][1][before + q] = h.y;
+	if (warp == kP - 1) {
+		S.half[b][0][total + lane] = S.half[b][1][total + lane] = 0.0f;
+		if (lane == 0) S.meta[b].x = total;
 	}
-	if (tid == 0) {
-		S.meta[b].x = total;
-		S.meta[b].z = own;
+#pragma unroll
+	for (int i = 0; i < R; ++i)
+		if (i * kWarp + lane < cnt) place(cd[i], h[i], before + i * kWarp + lane);
+	for (int q = R * kWarp + lane; q < cnt; q += kWarp) {
+		const float4 c = cand[q];
+		const float2 hh = delta_half(make_float2(c.y, c.z), xk, c.w, pk, s);
+		if (c.w >= 0.0f) apply(c, hh);
+		place(c, hh, before + q);
 	}
 }
 
