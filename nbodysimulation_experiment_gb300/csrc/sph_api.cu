@@ -87,6 +87,11 @@ struct Scene {
 	int cellBase = 0, pBase = 0, bodyBase = 0;  // offsets into the shared arrays
 	sph_spring_params springs{};
 	std::vector<float2> pendPos, pendForce;
+	// Runs of the particles added since the last update (appendix tasks): the
+	// number where the first begins, and where each ends.
+	size_t runFrom = 0;
+	std::vector<int> runEnd;
+	float2 runLast{};
 };
 
 }  // namespace
@@ -337,6 +342,38 @@ int ensure_stage(sph_sim *s, size_t count) {
 	return SPH_OK;
 }
 
+// Divide the `count` pending particles (numbers nDev onwards) into appendix
+// runs: kAppendixRun consecutive ones, or fewer where the next particle lies
+// far away, as at the end of a lattice row.  A run across that jump would have
+// a box as wide as the lattice: it would wait for, and hold up, every run of
+// two rows, and its region would outgrow the sweep's stage (30,011 particles
+// in rows of 174: delta sweep of the first update 26 against 7.8 ms).  At most one run per
+// sixteen particles in all, whatever their order.
+void extend_runs(Scene &sc, size_t count) {
+	if (sc.nDev == sc.n0) {
+		sc.runEnd.clear();
+		sc.runFrom = sc.n0;
+	}
+	if ((sc.runEnd.empty() ? sc.runFrom : (size_t)sc.runEnd.back()) != sc.nDev) return;  // unknown numbers: fixed runs
+	if (!sc.runEnd.empty()) sc.runEnd.pop_back();  // the last run goes on
+	size_t from = sc.runEnd.empty() ? sc.runFrom : (size_t)sc.runEnd.back();
+	const float far = 2.0f * sc.dom.cell_size;
+	float2 last = sc.nDev == sc.runFrom ? sc.pendPos[0] : sc.runLast;
+	for (size_t k = 0; k < count; ++k) {
+		const size_t i = sc.nDev + k;
+		const float2 p = sc.pendPos[k];
+		const bool jump = std::fabs(p.x - last.x) > far || std::fabs(p.y - last.y) > far;
+		if (i - from == (size_t)kAppendixRun ||
+		    (jump && i > from && (sc.runEnd.size() + 1) * (kAppendixRun / 2) <= i - sc.runFrom)) {
+			sc.runEnd.push_back((int)i);
+			from = i;
+		}
+		last = p;
+	}
+	sc.runLast = last;
+	sc.runEnd.push_back((int)(sc.nDev + count));
+}
+
 // Pending AddParticle calls reach the device in order, before anything that
 // reads or changes device state.
 int flush_adds(sph_sim *s) {
@@ -359,6 +396,7 @@ int flush_adds(sph_sim *s) {
 		    sc.pBase + (int)sc.nDev, (int)count, (int)k, (int)sc.nDev, s->stagePos, s->stageForce,
 		    s->buf[s->cur].view(), tables(s));
 		SPH_LAUNCHED(s);
+		extend_runs(sc, count);
 		sc.nDev += count;
 		sc.pendPos.clear();
 		sc.pendForce.clear();
@@ -438,38 +476,47 @@ int check_device_errors(sph_sim *s) {
 	return SPH_OK;
 }
 
-// Appendix runs (particles added since the last update, kAppendixRun at a
-// time) of every scene as delta-sweep tasks after the canonical ones,
+// Appendix runs (particles added since the last update, extend_runs) of every
+// scene as delta-sweep tasks after the canonical ones,
 // interleaved across scenes; in reference order, runs of the whole scene in
 // AddParticle order are the only delta-sweep tasks.  A run waits for the earlier runs of its scene
 // whose particles' new cells come within two cells of its own, so a scene's
 // appendix is relaxed as in AddParticle order.
 int upload_appendix_tasks(sph_sim *s) {
 	const size_t S = s->scenes.size();
-	std::vector<int> runs(S);
-	int maxRuns = 0;
+	std::vector<std::vector<int>> ends(S);  // per scene: where its runs end
+	std::vector<int> begin(S, 0);
+	size_t maxRuns = 0;
 	for (size_t k = 0; k < S; ++k) {
 		const Scene &sc = s->scenes[k];
 		// In reference order the delta sweep runs over the whole scene.
 		const size_t first = s->refOrder ? 0 : sc.n0;
-		runs[k] = (int)((sc.nDev - first + kAppendixRun - 1) / kAppendixRun);
-		maxRuns = std::max(maxRuns, runs[k]);
+		begin[k] = (int)first;
+		if (first == sc.nDev) continue;
+		if (!s->refOrder && sc.runFrom == first && !sc.runEnd.empty() && (size_t)sc.runEnd.back() == sc.nDev) {
+			ends[k] = sc.runEnd;
+		} else {
+			for (size_t e = first; e < sc.nDev;) ends[k].push_back((int)(e = std::min(e + kAppendixRun, sc.nDev)));
+		}
+		maxRuns = std::max(maxRuns, ends[k].size());
 	}
 	s->nApp = 0;
 	if (maxRuns == 0) return SPH_OK;
-	std::vector<int> scene, run;
-	for (int r = 0; r < maxRuns; ++r) {
+	std::vector<int> scene, from, to;
+	for (size_t r = 0; r < maxRuns; ++r) {
 		for (size_t k = 0; k < S; ++k) {
-			if (r >= runs[k]) continue;
+			if (r >= ends[k].size()) continue;
 			scene.push_back((int)k);
-			run.push_back(r);
+			from.push_back(r ? ends[k][r - 1] : begin[k]);
+			to.push_back(ends[k][r]);
 		}
 	}
 	if ((size_t)s->ncellTotal + scene.size() > s->doneDCap) return SPH_ERR_CAPACITY;
 	s->nApp = (int)scene.size();
 	const size_t bytes = scene.size() * sizeof(int);
 	SPH_CUDA(cudaMemcpyAsync(s->T.appScene, scene.data(), bytes, cudaMemcpyHostToDevice, s->stream));
-	SPH_CUDA(cudaMemcpyAsync(s->T.appRun, run.data(), bytes, cudaMemcpyHostToDevice, s->stream));
+	SPH_CUDA(cudaMemcpyAsync(s->T.appFrom, from.data(), bytes, cudaMemcpyHostToDevice, s->stream));
+	SPH_CUDA(cudaMemcpyAsync(s->T.appTo, to.data(), bytes, cudaMemcpyHostToDevice, s->stream));
 	return SPH_OK;
 }
 
@@ -774,12 +821,13 @@ int allocate(sph_sim *s) {
 	    (rc = dalloc(&T.nLive, 1)) ||
 	    (rc = dalloc(&T.abort, 1)) || (rc = dalloc(&T.bodies, s->bodyCap)))
 		return rc;
-	// Appendix runs: at most one partial run per scene beyond N / kAppendixRun.
-	const size_t appCap = (N + kAppendixRun - 1) / kAppendixRun + S + 1;
+	// Appendix runs (extend_runs): at most one per kAppendixRun / 2 particles of a
+	// scene, and two more.
+	const size_t appCap = N / (kAppendixRun / 2) + 2 * S + 1;
 	s->doneDCap = C + appCap;
 	// Viscosity done flags: one per cell, or per run in reference order.
 	if ((rc = dalloc(&s->doneD, s->doneDCap)) || (rc = dalloc(&T.appScene, appCap)) ||
-	    (rc = dalloc(&T.appRun, appCap)) || (rc = dalloc(&T.appBox, 4 * appCap)) ||
+	    (rc = dalloc(&T.appFrom, appCap)) || (rc = dalloc(&T.appTo, appCap)) || (rc = dalloc(&T.appBox, 4 * appCap)) ||
 	    (rc = dalloc(&s->doneV, std::max(C, appCap))) || (rc = dalloc(&T.refOrd, N)) ||
 	    (rc = dalloc(&T.viscBox, 4 * appCap)) || (rc = dalloc(&s->check, 4)))
 		return rc;
@@ -1366,7 +1414,7 @@ int sph_destroy(sph_sim *s) {
 	}
 	SimTables &T = s->T;
 	void *ptrs[] = {s->cellStartA, s->cellCountA, s->cellStartB, s->cellCountB, T.taskOfCell,  T.taskCell,
-	                T.numberOrder, T.sceneOfCell, T.sceneOf,     T.scenes,      T.appScene,    T.appRun,
+	                T.numberOrder, T.sceneOfCell, T.sceneOf,     T.scenes,      T.appScene,    T.appFrom,     T.appTo,
 	                T.appBox,      T.appCount,    T.appStart,    T.appIdx,      T.appCursor,   T.newCell,
 	                T.enterCount,  T.leaveCount,  T.enterOffset, T.enterCursor, T.enterList,   T.moverCount,
 	                T.bbox,        T.newIdx,      T.newLabel,    T.taskCounter, T.stats,       T.error,

@@ -33,7 +33,7 @@ constexpr int kRegionCells = 100;
 constexpr int kMaxBodies = 100;  // kSPHMaxBodyCount, sph.h:71
 constexpr int kMaxPoly = 8;      // kMaxScenarioPolygonCount, sph.h:161
 // Appendix particles (added since the last update) are swept serially in runs
-// of this many consecutive numbers.
+// of at most this many consecutive numbers.
 constexpr int kAppendixRun = 32;
 // Pending dependencies a delta-sweep task lists before one warp polls them.
 constexpr int kPendCap = 128;
@@ -132,7 +132,7 @@ struct SimTables {
 	int *numberOrder;                  // global cells in numbering order (scene-major, colour rank)
 	int *sceneOfCell, *sceneOf;        // scene of a global cell / of a particle number
 	SceneDev *scenes;
-	int *appScene, *appRun;            // appendix run tasks: scene, run within the scene
+	int *appScene, *appFrom, *appTo;   // appendix run tasks: scene, the run's particles within the scene
 	int *appBox;                       // per appendix run: x0, y0, x1, y1 of its particles' new cells
 	// Reference order: refOrd[pBase + id] = number of the particle with
 	// AddParticle index id; viscBox per viscosity run: x0, y0, x1, y1 of its

@@ -1549,8 +1549,7 @@ __global__ void k_app_boxes(Totals tt, SimTables T) {
 	if (a >= tt.nApp) return;
 	const SceneDev &sc = T.scenes[T.appScene[a]];
 	const int gx = sc.p.gx;
-	const int p0 = sc.pBase + (tt.refOrder ? 0 : sc.n0) + T.appRun[a] * kAppendixRun;
-	const int p1 = min(sc.pBase + sc.n, p0 + kAppendixRun);
+	const int p0 = sc.pBase + T.appFrom[a], p1 = sc.pBase + T.appTo[a];
 	int bx0 = sc.p.gx, by0 = sc.p.gy, bx1 = -1, by1 = -1;
 	for (int k = p0 + lane; k < p1; k += kWarp) {
 		const int lc = T.newCell[tt.refOrder ? T.refOrd[k] : k] - sc.cellBase;
@@ -2403,6 +2402,53 @@ __device__ __forceinline__ unsigned long long relax_group(DeltaSmemT<C> &S, int 
 	return tStaged;
 }
 
+// One more pending dependency per thread (its done flag's index, or -1) into
+// `pend`; collective over the warp.
+__device__ __forceinline__ void list_pending(int r, int *pend, int *npend, int lane) {
+	const unsigned m = __ballot_sync(kFull, r >= 0);
+	int base = 0;
+	if (lane == 0 && m != 0u) base = atomicAdd(npend, __popc(m));
+	base = __shfl_sync(kFull, base, 0);
+	if (r >= 0) {
+		const int k = base + __popc(m & lanemask_lt());
+		if (k < kPendCap) pend[k] = r;
+	}
+}
+
+// Warp 0 polls the listed dependencies.
+__device__ __forceinline__ void poll_pending(const int *pend, int np, const SimTables &T, int tid) {
+	if (tid >= kWarp) return;
+	for (int k0 = 0; k0 < np; k0 += kWarp)
+		warp_wait(k0 + tid < np ? &T.done[pend[k0 + tid]] : nullptr, T.abort, T.error, T.waitLimitNs);
+}
+
+// Wait for the runs before run `a` of the scene whose boxes come within two
+// cells of `box`, as wait_canonical does for cells.  Collective over the block.
+template <int kDT>
+__device__ __forceinline__ void wait_runs(int a, int scene, int4 box, const SimTables &T, int flag0, int *pend,
+                                          int *npend, int tid) {
+	if (tid == 0) *npend = 0;
+	__syncthreads();
+	auto near = [&](int q) {
+		if (q >= a || T.appScene[q] != scene) return false;
+		const int4 o = *reinterpret_cast<const int4 *>(&T.appBox[4 * q]);
+		return rect_dist(o.x, o.y, o.z, o.w, box.x, box.y, box.z, box.w) <= 2;
+	};
+	for (int q0 = 0; q0 < a; q0 += kDT) {
+		const int q = q0 + tid;
+		list_pending(near(q) && ld_acquire(&T.done[flag0 + q]) == 0u ? flag0 + q : -1, pend, npend, tid & (kWarp - 1));
+	}
+	__syncthreads();
+	const int np = *npend;
+	if (np > kPendCap) {
+		for (int q0 = 0; q0 < a; q0 += kDT)
+			warp_wait(near(q0 + tid) ? &T.done[flag0 + q0 + tid] : nullptr, T.abort, T.error, T.waitLimitNs);
+	} else {
+		poll_pending(pend, np, T, tid);
+	}
+	__syncthreads();
+}
+
 // Wait for canonical tasks of the scene (old cells) near [bx0,bx1]x[by0,by1]
 // whose new-cell bounding boxes come within two cells of it and whose task
 // index is below `limit`.  Collective over the block.  The block first
@@ -2435,14 +2481,7 @@ __device__ __forceinline__ void wait_canonical(int bx0, int by0, int bx1, int by
 				if (rect_dist(b.x, b.y, b.z, b.w, bx0, by0, bx1, by1) <= 2 && ld_acquire(&T.done[r2]) == 0u) r = r2;
 			}
 		}
-		const unsigned m = __ballot_sync(kFull, r >= 0);
-		int base = 0;
-		if (lane == 0 && m != 0u) base = atomicAdd(npend, __popc(m));
-		base = __shfl_sync(kFull, base, 0);
-		if (r >= 0) {
-			const int k = base + __popc(m & lanemask_lt());
-			if (k < kPendCap) pend[k] = r;
-		}
+		list_pending(r, pend, npend, lane);
 	}
 	__syncthreads();
 	const int np = *npend;
@@ -2461,9 +2500,8 @@ __device__ __forceinline__ void wait_canonical(int bx0, int by0, int bx1, int by
 			}
 			warp_wait(flag, T.abort, T.error, T.waitLimitNs);
 		}
-	} else if (tid < kWarp) {
-		for (int k0 = 0; k0 < np; k0 += kWarp)
-			warp_wait(k0 + lane < np ? &T.done[pend[k0 + lane]] : nullptr, T.abort, T.error, T.waitLimitNs);
+	} else {
+		poll_pending(pend, np, T, tid);
 	}
 	__syncthreads();
 }
@@ -2516,22 +2554,12 @@ __global__ void __launch_bounds__(C::kWarps * kWarp, C::kMinBlocks) k_delta(Tota
 			const SceneDev &sc = T.scenes[scene];
 			const StepParams s = sc.p;
 			const int base = sc.cellBase;
-			const int p0 = sc.pBase + (tt.refOrder ? 0 : sc.n0) + T.appRun[a] * kAppendixRun;
-			const int p1 = min(sc.pBase + sc.n, p0 + kAppendixRun);
+			const int p0 = sc.pBase + T.appFrom[a], p1 = sc.pBase + T.appTo[a];
 			const int4 box = *reinterpret_cast<const int4 *>(&T.appBox[4 * a]);
 			const int bx0 = box.x, by0 = box.y, bx1 = box.z, by1 = box.w;
 			if (!tt.refOrder)
 				wait_canonical<kDT>(bx0, by0, bx1, by1, moveMax, tt.ncell, -1, T, s, base, S.pend, &S.npend, tid);
-			for (int q0 = 0; q0 < a; q0 += kDT) {
-				const int q = q0 + tid;
-				const uint32_t *flag = nullptr;
-				if (q < a && T.appScene[q] == scene) {
-					const int4 o = *reinterpret_cast<const int4 *>(&T.appBox[4 * q]);
-					if (rect_dist(o.x, o.y, o.z, o.w, bx0, by0, bx1, by1) <= 2) flag = &T.done[tt.ncell + q];
-				}
-				warp_wait(flag, T.abort, T.error, T.waitLimitNs);
-			}
-			__syncthreads();
+			wait_runs<kDT>(a, scene, box, T, tt.ncell, S.pend, &S.npend, tid);
 			relax_group<C>(S, p0, p1, ord, bx0, by0, bx1, by1, Q, T, s, base, tid);
 			__syncthreads();
 			__threadfence();
