@@ -636,17 +636,22 @@ int enqueue_step(sph_sim *s, bool capturing) {
 	return SPH_OK;
 }
 
-// Viscosity pair lists longer than this send the lean viscosity shape's
-// chains through several rounds; the wide shape stays staged.
-constexpr uint32_t kDenseNeighbors = 440;
+// Where dense states change shapes: measured crossovers on the collapsing 1M
+// column, whose other scenes' lie no lower.  Viscosity, longest neighbour list
+// of 542: lean 4.12 against wide 4.31 ms, of 577: 4.66 against 4.33.
+constexpr uint32_t kDenseNeighbors = 555;
+// Delta sweep, fullest cell of 117 particles: quad 3.97 against mid 4.10 ms, of
+// 138: 5.12 against 4.73 (tri from about 100).
+constexpr uint32_t kDenseCell = 120;
+// Fullest cell of 139: mid 6.21 against dense 6.29, of 162: 7.52 against 7.11.
+constexpr uint32_t kCrowdedCell = 145;
 
 // The sweep shapes of the next update: the tuned ones, or in dense states
-// (see sph_sim::adaptive) the wide viscosity shape and a delta shape whose
-// stage holds the task regions: the 8-warp shape (4,096 entries) once a 3x3
-// block of the fullest cell passes 0.65 of the tuned shape's stage, the
-// 16-warp shape (12,288 entries) once a 5x5 region of it nears 4,096.  The statistics are those of the update
-// before last at the latest: the host waits for its copy, so it never runs
-// more than two updates ahead.  Changing shapes drops the update graphs.
+// (see sph_sim::adaptive) the wide viscosity shape and, where the tuned delta
+// shape's stage is smaller, the 8-warp shape (4,096 entries) or, more crowded
+// still, the 16-warp shape (12,288 entries).  The statistics are those of the
+// update before last at the latest: the host waits for its copy, so it never
+// runs more than two updates ahead.  Changing shapes drops the update graphs.
 void choose_shapes(sph_sim *s) {
 	int vl = s->viscLean, vb = s->viscBlocks, ds = s->deltaShape, db = s->deltaBlocks;
 	// A batch of many scenes keeps its tuned shapes: its sweeps are bound by
@@ -664,15 +669,8 @@ void choose_shapes(sph_sim *s) {
 		// Hysteresis: back to the tuned shape only well below the threshold.
 		s->denseVisc = s->denseVisc ? maxNb * 5 > kDenseNeighbors * 4 : maxNb > kDenseNeighbors;
 		const uint32_t cap = (uint32_t)delta_stage_capacity(ds);
-		const uint32_t block = 9 * maxCell;   // a 3x3 block at the fullest cell's count
-		const uint32_t spread = 25 * maxCell;  // a 5x5 region: a cell's particles spread over 3x3 new cells
-		// Thresholds from measured crossovers on the collapsing 1M column:
-		// the 8-warp shape wins from ~110 particles in the fullest cell (a
-		// 3x3 block at 0.65 of the 1,536-entry stage), the 16-warp one from
-		// ~160 (a 5x5 region near 4,096).
-		s->denseDelta = s->denseDelta ? block * 2 > cap : block * 20 > cap * 13;
-		s->crowdedDelta =
-		    s->crowdedDelta ? spread * 5 > (uint32_t)kDeltaStageCap * 4 : spread * 20 > (uint32_t)kDeltaStageCap * 19;
+		s->denseDelta = maxCell * (s->denseDelta ? 5u : 4u) > kDenseCell * 4u;
+		s->crowdedDelta = maxCell * (s->crowdedDelta ? 5u : 4u) > kCrowdedCell * 4u;
 		if (vl && s->denseVisc) {
 			vl = 0;
 			vb = s->denseViscBlocks;

@@ -47,7 +47,7 @@ struct DeltaWide {
 };
 struct DeltaLean {
 	static constexpr int kName = 2;
-	static constexpr int kWarps = 2, kProducers = 1, kStage = 1536, kChainW = 192, kPrefetch = 64, kMinBlocks = 8;
+	static constexpr int kWarps = 2, kProducers = 1, kStage = 1760, kChainW = 192, kPrefetch = 64, kMinBlocks = 8;
 	static constexpr int kRegion = kRegionCells;
 	static constexpr bool kPipelined = false, kShortEntry = false, kDirect = false, kApart = false;
 };
@@ -64,13 +64,13 @@ struct DeltaMid {
 // three (quad) producer warps and the summer warp, several blocks per SM.
 struct DeltaTri {
 	static constexpr int kName = 3;
-	static constexpr int kWarps = 3, kProducers = 2, kStage = 1536, kChainW = 256, kPrefetch = 64, kMinBlocks = 5;
+	static constexpr int kWarps = 3, kProducers = 2, kStage = 2000, kChainW = 256, kPrefetch = 64, kMinBlocks = 5;
 	static constexpr int kRegion = kRegionCells;
 	static constexpr bool kPipelined = true, kShortEntry = true, kDirect = false, kApart = false;
 };
 struct DeltaQuad {
 	static constexpr int kName = 4;
-	static constexpr int kWarps = 4, kProducers = 3, kStage = 1536, kChainW = 192, kPrefetch = 128, kMinBlocks = 4;
+	static constexpr int kWarps = 4, kProducers = 3, kStage = 3072, kChainW = 192, kPrefetch = 128, kMinBlocks = 4;
 	static constexpr int kRegion = kRegionCells;
 	static constexpr bool kPipelined = true, kShortEntry = true, kDirect = false, kApart = true;
 };
