@@ -197,8 +197,8 @@ int backward(sph_mpnn *m, const MpnnGraph &G, const float2 *target, cudaStream_t
 		MPNN_CUDA(cudaGetLastError());
 		dim3 tg(blocks(kHidden, 32), blocks(np, 32));
 		k_mpnn_transpose<<<tg, dim3(32, 8), 0, st>>>(m->da3b, np, kHidden, kHidden, m->da3f, np);
-		k_mpnn_dw4<<<kHidden, 256, 0, st>>>(dzNext, m->cf[r], np, n, Gp + kOffW4, Gp + kOffB4);
-		k_mpnn_rowsum<<<kHidden, 256, 0, st>>>(m->da3f, np, n, nullptr, Gp + kOffB3);
+		k_mpnn_dw4<<<dim3(kHidden, kReduceParts), kReduceThreads, 0, st>>>(dzNext, m->cf[r], np, n, Gp + kOffW4, Gp + kOffB4);
+		k_mpnn_rowsum<<<dim3(kHidden, kReduceParts), kReduceThreads, 0, st>>>(m->da3f, np, n, nullptr, Gp + kOffB3);
 		MPNN_CUDA(cudaGetLastError());
 		// dW3 += da3^T X3 (reduction over particles).
 		GemmArgs g3 = gemm(m->da3f, np, m->X3f[r], np, kHidden, kNodeInPad, np, m->error);
@@ -218,7 +218,7 @@ int backward(sph_mpnn *m, const MpnnGraph &G, const float2 *target, cudaStream_t
 		g4.ldcbT = np;
 		rc = run_gemm(g4, 1, st);
 		if (rc) return rc;
-		k_mpnn_rowsum<<<kHidden, 256, 0, st>>>(m->dXf, np, n, m->degS, Gp + kOffB2);
+		k_mpnn_rowsum<<<dim3(kHidden, kReduceParts), kReduceThreads, 0, st>>>(m->dXf, np, n, m->degS, Gp + kOffB2);
 		MPNN_CUDA(cudaGetLastError());
 		// dW2 += dM^T H.
 		GemmArgs g5 = gemm(m->dXf, np, m->Hf[r], np, kHidden, kHidden, np, m->error);
@@ -237,7 +237,7 @@ int backward(sph_mpnn *m, const MpnnGraph &G, const float2 *target, cudaStream_t
 		MpnnGraph Gr = G;
 		const int needDz = r > 0;
 		if (needDz) MPNN_CUDA(cudaMemsetAsync(m->dzEdge, 0, sizeof(float2) * np, st));
-		k_mpnn_edge_bwd<<<edge_blocks(G), kEdgeWarps * kWarp, mpnn_edge_smem(true), st>>>(
+		k_mpnn_edge_bwd<<<std::min(G.gx * G.gy, 4 * 2 * m->sms), kBwdWarps * kWarp, mpnn_edge_smem(true), st>>>(
 		    Gr, P + kOffW1, P + kOffB1, zr, m->dH, m->dzEdge, Gp + kOffW1, Gp + kOffB1, needDz, m->error);
 		MPNN_CUDA(cudaGetLastError());
 		if (needDz) {

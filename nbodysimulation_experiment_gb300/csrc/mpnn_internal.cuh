@@ -80,6 +80,9 @@ struct MpnnGraph {
 };
 
 constexpr int kEdgeWarps = 4;
+constexpr int kBwdWarps = 8;        // k_mpnn_edge_bwd: warps sharing a cell's staged block
+constexpr int kReduceThreads = 256;  // row sums over the particles
+constexpr int kReduceParts = 8;      // blocks per row
 size_t mpnn_edge_smem(bool backward);
 size_t mpnn_edge_tc_smem();
 int mpnn_edge_tc_blocks_per_sm();
