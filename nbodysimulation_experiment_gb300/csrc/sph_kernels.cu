@@ -1811,61 +1811,48 @@ __device__ __forceinline__ bool stage_table(DeltaSmemT<C> &S, Region &R, const S
 	return R.L <= C::kStage;
 }
 
-// Stage the table's positions.  Collective over the block.
+// Stage the table's positions, a warp per cell, the loads of kStageCells cells
+// (64 entries each) in flight at once.  Collective over the block.  (One entry
+// per thread, its cell found by binary search over the table's offsets: 768 ns
+// in the wide shape and 5.4 us in the lean one for 25 cells of 36 particles, now
+// 320 ns and 2.6 us; one cell at a time 480 ns and 4.1 us; four, with registers
+// spilled around the pipeline, slowed the particles by a tenth.)
+constexpr int kStageCells = 2;
 template <class C>
 __device__ __forceinline__ void stage_positions(DeltaSmemT<C> &S, const Region &R, const Particles &Q, int tid) {
-	constexpr int kDT = C::kWarps * kWarp;
-	for (int b0 = 0; b0 < R.L; b0 += 4 * kDT) {
-		float2 xp[4];
+	const int lane = tid & (kWarp - 1);
+	for (int q0 = tid / kWarp; q0 < R.ncells; q0 += kStageCells * C::kWarps) {
+		float2 xp[kStageCells][2];
+		int off[kStageCells], n[kStageCells], st[kStageCells];
 #pragma unroll
-		for (int u = 0; u < 4; ++u) {
-			const int e = b0 + u * kDT + tid;
-			if (e < R.L) {
-				int lo = 0, hi = R.ncells;
-				while (hi - lo > 1) {
-					const int mid = (lo + hi) >> 1;
-					if (S.segOff[mid] <= e) lo = mid; else hi = mid;
-				}
-				xp[u] = __ldcg(&Q.pos[S.segStart[lo] + (e - S.segOff[lo])]);
-			}
+		for (int u = 0; u < kStageCells; ++u) {
+			const int q = min(q0 + u * C::kWarps, R.ncells - 1);
+			off[u] = S.segOff[q];
+			n[u] = q0 + u * C::kWarps < R.ncells ? S.segOff[q + 1] - off[u] : 0;
+			st[u] = S.segStart[q];
+#pragma unroll
+			for (int v = 0; v < 2; ++v)
+				if (v * kWarp + lane < n[u]) xp[u][v] = __ldcg(&Q.pos[st[u] + v * kWarp + lane]);
 		}
 #pragma unroll
-		for (int u = 0; u < 4; ++u) {
-			const int e = b0 + u * kDT + tid;
-			if (e < R.L) S.pos[e] = xp[u];
+		for (int u = 0; u < kStageCells; ++u) {
+#pragma unroll
+			for (int v = 0; v < 2; ++v)
+				if (v * kWarp + lane < n[u]) S.pos[off[u] + v * kWarp + lane] = xp[u][v];
+			for (int j = 2 * kWarp + lane; j < n[u]; j += kWarp) S.pos[off[u] + j] = __ldcg(&Q.pos[st[u] + j]);
 		}
 	}
 	__syncthreads();
 }
 
-// Write the staged positions of the owned cells back.  Flat: one element
-// per thread, its cell found by binary search over the region's offsets as
-// in staging, so no thread walks the cells one after another.  Otherwise
-// cell by cell, with fewer instructions per element.
+// Write the staged positions of the owned cells back, a warp per cell.
 template <class C>
 __device__ __forceinline__ void write_back_owned(DeltaSmemT<C> &S, const Region &R, const Particles &Q, int tid) {
-	constexpr int kDT = C::kWarps * kWarp;
-	if constexpr (!C::kShortEntry) {
-		for (int q = 0; q < R.ncells; ++q) {
-			if (!S.owned[q]) continue;
-			const int off = S.segOff[q], nn = S.segOff[q + 1] - off, st = S.segStart[q];
-			for (int j = tid; j < nn; j += kDT) __stcg(&Q.pos[st + j], S.pos[off + j]);
-		}
-	} else {
-		for (int b0 = 0; b0 < R.L; b0 += 4 * kDT) {
-#pragma unroll
-			for (int u = 0; u < 4; ++u) {
-				const int e = b0 + u * kDT + tid;
-				if (e < R.L) {
-					int lo = 0, hi = R.ncells;
-					while (hi - lo > 1) {
-						const int mid = (lo + hi) >> 1;
-						if (S.segOff[mid] <= e) lo = mid; else hi = mid;
-					}
-					if (S.owned[lo]) __stcg(&Q.pos[S.segStart[lo] + (e - S.segOff[lo])], S.pos[e]);
-				}
-			}
-		}
+	const int lane = tid & (kWarp - 1);
+	for (int q = tid / kWarp; q < R.ncells; q += C::kWarps) {
+		if (!S.owned[q]) continue;
+		const int off = S.segOff[q], n = S.segOff[q + 1] - off, st = S.segStart[q];
+		for (int j = lane; j < n; j += kWarp) __stcg(&Q.pos[st + j], S.pos[off + j]);
 	}
 }
 

@@ -29,27 +29,24 @@ struct ViscLean {
 // in the pipeline when it has at most kProducers * kChainW entries.  kName
 // names the shape in sph_set_sweep_shape.  Wide: twelve producers, one block
 // per SM (short per-particle latency for one scene).  Lean: two warps, not
-// pipelined, smaller staging (more tasks per SM for many scenes).
-// kShortEntry: a task's entry and exit take the fewest cycles (first chunk's
-// inputs loaded during the staging, region written back one element per
-// thread) rather than the fewest instructions.  kDirect: a producer thread
-// evaluates the list entries it scans itself (shortest phase, for the shapes
-// with many warps per task); otherwise the in-range entries are compacted
-// first (fewest square roots and divisions, for the shapes with two or three
-// producer warps: evaluated directly, tri took 1,853 ns per particle of one
-// task alone against 1,445, quad 1,234 against 1,148).  kApart: the summer has
-// its scheduler to itself (pipeline_role).
+// pipelined, smaller staging (more tasks per SM for many scenes).  kDirect: a
+// producer thread evaluates the list entries it scans itself (shortest phase,
+// for the shapes with many warps per task); otherwise the in-range entries are
+// compacted first (fewest square roots and divisions, for the shapes with two
+// or three producer warps: evaluated directly, tri took 1,853 ns per particle
+// of one task alone against 1,445, quad 1,234 against 1,148).  kApart: the
+// summer has its scheduler to itself (pipeline_role).
 struct DeltaWide {
 	static constexpr int kName = 12;
 	static constexpr int kWarps = 16, kProducers = 12, kStage = kDeltaStageCap, kChainW = 96, kPrefetch = 128, kMinBlocks = 1;
 	static constexpr int kRegion = kRegionCells;
-	static constexpr bool kPipelined = true, kShortEntry = true, kDirect = true, kApart = true;
+	static constexpr bool kPipelined = true, kDirect = true, kApart = true;
 };
 struct DeltaLean {
 	static constexpr int kName = 2;
 	static constexpr int kWarps = 2, kProducers = 1, kStage = 1760, kChainW = 192, kPrefetch = 64, kMinBlocks = 8;
 	static constexpr int kRegion = kRegionCells;
-	static constexpr bool kPipelined = false, kShortEntry = false, kDirect = false, kApart = false;
+	static constexpr bool kPipelined = false, kDirect = false, kApart = false;
 };
 // Mid: pipelined, six producers, two blocks per SM (mid-size scenes, where
 // more tasks run at once than one block per SM holds).
@@ -57,7 +54,7 @@ struct DeltaMid {
 	static constexpr int kName = 8;
 	static constexpr int kWarps = 8, kProducers = 6, kStage = kDeltaStageCap, kChainW = 160, kPrefetch = 128, kMinBlocks = 2;
 	static constexpr int kRegion = 256;
-	static constexpr bool kPipelined = true, kShortEntry = true, kDirect = true, kApart = true;
+	static constexpr bool kPipelined = true, kDirect = true, kApart = true;
 };
 // Small pipelined shapes for large scenes, where the sweep is bound by how
 // many tasks run at once rather than by one task's latency: two (tri) or
@@ -66,13 +63,13 @@ struct DeltaTri {
 	static constexpr int kName = 3;
 	static constexpr int kWarps = 3, kProducers = 2, kStage = 2000, kChainW = 256, kPrefetch = 64, kMinBlocks = 5;
 	static constexpr int kRegion = kRegionCells;
-	static constexpr bool kPipelined = true, kShortEntry = true, kDirect = false, kApart = false;
+	static constexpr bool kPipelined = true, kDirect = false, kApart = false;
 };
 struct DeltaQuad {
 	static constexpr int kName = 4;
 	static constexpr int kWarps = 4, kProducers = 3, kStage = 3072, kChainW = 192, kPrefetch = 128, kMinBlocks = 4;
 	static constexpr int kRegion = kRegionCells;
-	static constexpr bool kPipelined = true, kShortEntry = true, kDirect = false, kApart = true;
+	static constexpr bool kPipelined = true, kDirect = false, kApart = true;
 };
 // Dense: pipelined, twelve producers, one block per SM, a 12,288-entry stage,
 // for crowded states where a task's region (the bounding box of its
@@ -82,7 +79,7 @@ struct DeltaDense {
 	static constexpr int kName = 16;
 	static constexpr int kWarps = 16, kProducers = 12, kStage = kDeltaDenseStageCap, kChainW = 96, kPrefetch = 128, kMinBlocks = 1;
 	static constexpr int kRegion = 400;
-	static constexpr bool kPipelined = true, kShortEntry = true, kDirect = true, kApart = true;
+	static constexpr bool kPipelined = true, kDirect = true, kApart = true;
 };
 // Delta shapes by index (sph_set_sweep_shape names them by warp count).
 constexpr int kDeltaShapes = 6;
