@@ -101,6 +101,7 @@ struct sph_sim {
 	cudaStream_t stream = nullptr;
 	int numSMs = 0;
 	int viscBlocks = 0, deltaBlocks = 0, densBlocks = 0, gridBlocks = 0;
+	int densSplit = 0;  // two warps per cell, see k_density
 	int viscLean = 0;   // viscosity shape: 0 = wide, 1 = lean (sph_kernels.cuh)
 	bool refOrder = false;  // sweeps and grid events in AddParticle order (sph_set_reference_order)
 	int viscRefBlocks = 0;
@@ -609,7 +610,7 @@ int enqueue_step(sph_sim *s, bool capturing) {
 	}
 	SPH_CUDA(mark(kEvSprings));
 
-	k_density<<<s->densBlocks, kDensWarps * kWarp, dens_smem_bytes(), st>>>(tt, B.view(), T);
+	k_density<<<s->densBlocks, kDensWarps * kWarp, dens_smem_bytes(), st>>>(tt, B.view(), T, s->densSplit);
 	SPH_LAUNCHED(s);
 	SPH_CUDA(mark(kEvDensity));
 
@@ -905,7 +906,8 @@ int allocate(sph_sim *s) {
 		if (sweep_occupancy(false, kDeltaDense, &v2, &d2) != cudaSuccess || d2 < 1) return SPH_ERR_CUDA;
 		s->crowdedDeltaBlocks = d2 * s->numSMs;
 	}
-	s->densBlocks = std::max(1, std::min(blocks_for(C, kDensWarps), 64 * s->numSMs));
+	s->densSplit = C <= 112 * s->numSMs ? 1 : 0;
+	s->densBlocks = std::max(1, std::min(blocks_for(C << s->densSplit, kDensWarps), 64 * s->numSMs));
 	s->springBlocks = std::max(1, std::min(blocks_for(C, kSpringWarps), 64 * s->numSMs));
 	s->gridBlocks = std::max(1, std::min(blocks_for(C, kGridWarps), 64 * s->numSMs));
 	s->viscRefBlocks = 8 * s->numSMs;
@@ -1114,7 +1116,7 @@ int density_error(sph_sim *s, float *out, uint32_t *maxNb = nullptr) {
 	Particles Q = s->buf[s->cur].view();
 	Q.dens = s->ldens;
 	Q.press = s->lbyId;
-	k_density<<<s->densBlocks, kDensWarps * kWarp, dens_smem_bytes(), s->stream>>>(tt, Q, T);
+	k_density<<<s->densBlocks, kDensWarps * kWarp, dens_smem_bytes(), s->stream>>>(tt, Q, T, s->densSplit);
 	SPH_LAUNCHED(s);
 	const int blocks = std::min(blocks_for(tt.n, kErrThreads), kErrBlocks);
 	k_density_error<<<blocks, kErrThreads, 0, s->stream>>>(tt.n, s->ldens, sc.params.rest_density, s->lerr);

@@ -1598,10 +1598,21 @@ __global__ void k_app_boxes(Totals tt, SimTables T) {
 
 // ---------------------------------------------------------------------------
 // Density and pressure (demo4.cpp:208-221): a pure gather.  One warp per new
-// cell; each lane sums the lists of two of the cell's particles (the 3x3
+// cell; each lane sums the lists of up to two of the cell's particles (the 3x3
 // block of the new cell arrays, demo4.cpp:183-206) in list order.  The block
 // is staged in chunks of kDensChunk entries, so a warp needs little shared
 // memory and many warps fit on an SM.
+//
+// Bound by instruction issue on large grids (1M block: 0.78 instructions per
+// cycle and scheduler, DRAM 0.3 %), so a cell, or the rest of one, of at most
+// 32 particles runs the loop with one list per lane instead of an empty second
+// one (128 scenes 0.81 -> 0.71 ms, 1M block 0.44 -> 0.43).  Small grids are
+// bound by one warp's time for its cell; with `split` two warps share a cell,
+// 32 particles each at a time: 4,096 dam break 52 -> 35 us, 65,536 particles
+// among obstacles 99 -> 66 us, where on the 1M block the staging done twice
+// costs more (0.43 -> 0.49 ms).  The host splits while two warps for each
+// occupied cell, about one cell in seven of the scenes here, are resident at
+// once at 32 warps per SM: 112 cells per SM.
 
 constexpr int kDensChunk = 256;
 struct DensWarp {
@@ -1622,16 +1633,64 @@ __device__ __forceinline__ void dens_entry(float2 xj, float2 xi, float h2, float
 	}
 }
 
+// Lists of N particles per lane, j0 + 32 n in the cell at st with cnt
+// particles, over the L entries of its 3x3 block.
+template <int N>
+__device__ __forceinline__ void dens_lists(DensWarp &S, const Particles &Q, const int (&segOff)[9],
+                                           const int (&segStart)[9], int L, int st, int j0, int cnt,
+                                           const StepParams &s, int lane) {
+	const float h2 = s.h2, invH = s.invH;
+	float2 xi[N];
+	float d0[N], d1[N];
+#pragma unroll
+	for (int n = 0; n < N; ++n) {
+		const int j = j0 + n * kWarp;
+		// Lanes without a particle use a position no entry is in range of.
+		xi[n] = j < cnt ? Q.pos[st + j] : make_float2(3.0e38f, 3.0e38f);
+		d0[n] = d1[n] = 0.0f;
+	}
+	for (int c0 = 0; c0 < L; c0 += kDensChunk) {
+		const int len = min(kDensChunk, L - c0);
+		__syncwarp();
+		for (int e = lane; e < len; e += kWarp) S.pos[e] = Q.pos[seg_src<9>(c0 + e, segOff, segStart)];
+		__syncwarp();
+		int e = 0;
+		for (; e + 4 <= len; e += 4) {
+			float2 xj[4];
+#pragma unroll
+			for (int u = 0; u < 4; ++u) xj[u] = S.pos[e + u];
+#pragma unroll
+			for (int u = 0; u < 4; ++u)
+#pragma unroll
+				for (int n = 0; n < N; ++n) dens_entry(xj[u], xi[n], h2, invH, d0[n], d1[n]);
+		}
+		for (; e < len; ++e) {
+			const float2 xj = S.pos[e];
+#pragma unroll
+			for (int n = 0; n < N; ++n) dens_entry(xj, xi[n], h2, invH, d0[n], d1[n]);
+		}
+	}
+#pragma unroll
+	for (int n = 0; n < N; ++n) {
+		const int j = j0 + n * kWarp;
+		if (j < cnt) {
+			Q.dens[st + j] = make_float2(d0[n], d1[n]);
+			Q.press[st + j] = make_float2(s.k * (d0[n] - s.rho0), s.kNear * d1[n]);
+		}
+	}
+}
+
 }  // namespace
 
-__global__ void __launch_bounds__(kDensWarps * kWarp, 4) k_density(Totals tt, Particles Q, SimTables T) {
+__global__ void __launch_bounds__(kDensWarps * kWarp, 4) k_density(Totals tt, Particles Q, SimTables T, int split) {
 	extern __shared__ __align__(16) unsigned char smem_raw[];
 	DensWarp &S = reinterpret_cast<DensWarp *>(smem_raw)[threadIdx.x / kWarp];
 	const int lane = threadIdx.x & (kWarp - 1);
 	const int warpsTotal = gridDim.x * kDensWarps;
-	for (int c = blockIdx.x * kDensWarps + threadIdx.x / kWarp; c < tt.ncell; c += warpsTotal) {
+	for (int w = blockIdx.x * kDensWarps + threadIdx.x / kWarp; w < tt.ncell << split; w += warpsTotal) {
+		const int c = w >> split, first = (w & split) * kWarp;
 		const int cnt = T.newCount[c];
-		if (cnt == 0) continue;
+		if (cnt <= first) continue;
 		const int sid = T.sceneOfCell[c];
 		const SceneDev &sc = T.scenes[sid];
 		const StepParams &s = sc.p;
@@ -1652,7 +1711,7 @@ __global__ void __launch_bounds__(kDensWarps * kWarp, 4) k_density(Totals tt, Pa
 			segOff[q] = L;
 			L += nn;
 		}
-		if (lane == 0) {
+		if (lane == 0 && first == 0) {
 			atomicMin(&T.stats[4 * sid + 0], (uint32_t)L);
 			atomicMax(&T.stats[4 * sid + 1], (uint32_t)L);
 		}
@@ -1660,45 +1719,12 @@ __global__ void __launch_bounds__(kDensWarps * kWarp, 4) k_density(Totals tt, Pa
 			if (lane == 0) atomicOr(T.error, kErrStageOverflow);
 			continue;
 		}
-		const float h2 = s.h2, invH = s.invH;
 		const int st = T.newStart[c];
-		for (int g = 0; g < cnt; g += 2 * kWarp) {
-			const int j0 = g + lane, j1 = g + kWarp + lane;
-			// Lanes without a particle use a position no entry is in range of.
-			const float2 far = make_float2(3.0e38f, 3.0e38f);
-			const float2 xi0 = j0 < cnt ? Q.pos[st + j0] : far;
-			const float2 xi1 = j1 < cnt ? Q.pos[st + j1] : far;
-			float d00 = 0.0f, d01 = 0.0f, d10 = 0.0f, d11 = 0.0f;
-			for (int c0 = 0; c0 < L; c0 += kDensChunk) {
-				const int n = min(kDensChunk, L - c0);
-				__syncwarp();
-				for (int e = lane; e < n; e += kWarp) S.pos[e] = Q.pos[seg_src<9>(c0 + e, segOff, segStart)];
-				__syncwarp();
-				int e = 0;
-				for (; e + 4 <= n; e += 4) {
-					float2 xj[4];
-#pragma unroll
-					for (int u = 0; u < 4; ++u) xj[u] = S.pos[e + u];
-#pragma unroll
-					for (int u = 0; u < 4; ++u) {
-						dens_entry(xj[u], xi0, h2, invH, d00, d01);
-						dens_entry(xj[u], xi1, h2, invH, d10, d11);
-					}
-				}
-				for (; e < n; ++e) {
-					const float2 xj = S.pos[e];
-					dens_entry(xj, xi0, h2, invH, d00, d01);
-					dens_entry(xj, xi1, h2, invH, d10, d11);
-				}
-			}
-			if (j0 < cnt) {
-				Q.dens[st + j0] = make_float2(d00, d01);
-				Q.press[st + j0] = make_float2(s.k * (d00 - s.rho0), s.kNear * d01);
-			}
-			if (j1 < cnt) {
-				Q.dens[st + j1] = make_float2(d10, d11);
-				Q.press[st + j1] = make_float2(s.k * (d10 - s.rho0), s.kNear * d11);
-			}
+		for (int g = first; g < cnt; g += 2 * kWarp) {
+			if (split == 0 && cnt - g > kWarp)
+				dens_lists<2>(S, Q, segOff, segStart, L, st, g + lane, cnt, s, lane);
+			else
+				dens_lists<1>(S, Q, segOff, segStart, L, st, g + lane, cnt, s, lane);
 		}
 		__syncwarp();
 	}
