@@ -539,15 +539,17 @@ int enqueue_step(sph_sim *s, bool capturing) {
 	};
 
 	SPH_CUDA(mark(kEvBegin));
-	k_integrate<<<blocks_for(cellOrN, kElemThreads), kElemThreads, 0, st>>>(tt, A.view(), T);
+	const int nDoneV = anyCanonical ? (tt.refOrder ? tt.nViscRuns : tt.ncell) : 0;
+	k_integrate<<<blocks_for(cellOrN, kElemThreads), kElemThreads, 0, st>>>(tt, A.view(), T, s->doneV, nDoneV,
+	                                                                        s->doneD, tt.ncell + tt.nApp);
 	SPH_LAUNCHED(s);
 	{
 		// The sweeps' task list: occupied canonical cells in task order.
 		const int ntiles = (tt.ncell + kScanTile - 1) / kScanTile;
-		k_live_reduce<<<ntiles, kScanThreads, 0, st>>>(tt, T);
-		SPH_LAUNCHED(s);
-		k_live_tiles<<<1, kScanThreads, 0, st>>>(T, ntiles);
-		SPH_LAUNCHED(s);
+		if (ntiles > 1) {
+			k_live_reduce<<<ntiles, kScanThreads, 0, st>>>(tt, T);
+			SPH_LAUNCHED(s);
+		}
 		k_live_apply<<<ntiles, kScanThreads, 0, st>>>(tt, T);
 		SPH_LAUNCHED(s);
 	}
@@ -558,8 +560,6 @@ int enqueue_step(sph_sim *s, bool capturing) {
 		SPH_LAUNCHED(s);
 	}
 	if (anyCanonical && tt.refOrder) {
-		SPH_CUDA(cudaMemsetAsync(s->doneV, 0, sizeof(uint32_t) * std::max(tt.nViscRuns, 1), st));
-		SPH_CUDA(cudaMemsetAsync(T.taskCounter, 0, sizeof(int), st));
 		SimTables v = T;
 		v.done = s->doneV;
 		k_visc_boxes<<<blocks_for((size_t)tt.nViscRuns * kWarp, kElemThreads), kElemThreads, 0, st>>>(tt, A.view(),
@@ -568,8 +568,6 @@ int enqueue_step(sph_sim *s, bool capturing) {
 		k_viscosity_ref<<<s->viscRefBlocks, kViscRefWarps * kWarp, 0, st>>>(tt, A.view(), v);
 		SPH_LAUNCHED(s);
 	} else if (anyCanonical) {
-		SPH_CUDA(cudaMemsetAsync(s->doneV, 0, sizeof(uint32_t) * s->ncellTotal, st));
-		SPH_CUDA(cudaMemsetAsync(T.taskCounter, 0, sizeof(int), st));
 		SimTables v = T;
 		v.done = s->doneV;
 		launch_viscosity(s->runViscLean != 0, s->runViscBlocks, st, tt, A.view(), v);
@@ -583,10 +581,10 @@ int enqueue_step(sph_sim *s, bool capturing) {
 
 	{
 		const int ntiles = (tt.ncell + kScanTile - 1) / kScanTile;
-		k_scan_reduce<<<ntiles, kScanThreads, 0, st>>>(tt, T);
-		SPH_LAUNCHED(s);
-		k_scan_tiles<<<1, kScanThreads, 0, st>>>(tt, T, ntiles);
-		SPH_LAUNCHED(s);
+		if (ntiles > 1) {
+			k_scan_reduce<<<ntiles, kScanThreads, 0, st>>>(tt, T);
+			SPH_LAUNCHED(s);
+		}
 		k_scan_apply<<<ntiles, kScanThreads, 0, st>>>(tt, T);
 		SPH_LAUNCHED(s);
 	}
@@ -618,8 +616,6 @@ int enqueue_step(sph_sim *s, bool capturing) {
 		k_app_boxes<<<blocks_for((size_t)tt.nApp * kWarp, kElemThreads), kElemThreads, 0, st>>>(tt, T);
 		SPH_LAUNCHED(s);
 	}
-	SPH_CUDA(cudaMemsetAsync(s->doneD, 0, sizeof(uint32_t) * (s->ncellTotal + s->nApp), st));
-	SPH_CUDA(cudaMemsetAsync(T.taskCounter + 1, 0, sizeof(int), st));
 	{
 		SimTables d = T;
 		d.done = s->doneD;

@@ -121,16 +121,15 @@ void launch_delta(int shape, int blocks, cudaStream_t st, Totals tt, Particles Q
 size_t dens_smem_bytes();
 size_t springs_smem_bytes();
 
-__global__ void k_integrate(Totals tt, Particles P, SimTables T);
+__global__ void k_integrate(Totals tt, Particles P, SimTables T, uint32_t *doneV, int nDoneV, uint32_t *doneD,
+                            int nDoneD);
 __global__ void k_ref_order(Totals tt, Particles P, SimTables T);
 __global__ void k_visc_boxes(Totals tt, Particles P, SimTables T);
 __global__ void k_viscosity_ref(Totals tt, Particles P, SimTables T);
 __global__ void k_predict(Totals tt, Particles P, SimTables T);
 __global__ void k_live_reduce(Totals tt, SimTables T);
-__global__ void k_live_tiles(SimTables T, int ntiles);
 __global__ void k_live_apply(Totals tt, SimTables T);
 __global__ void k_scan_reduce(Totals tt, SimTables T);
-__global__ void k_scan_tiles(Totals tt, SimTables T, int ntiles);
 __global__ void k_scan_apply(Totals tt, SimTables T);
 __global__ void k_scatter(Totals tt, Particles P, SimTables T);
 __global__ void k_grid_update(Totals tt, Particles P, Particles Q, SimTables T);
