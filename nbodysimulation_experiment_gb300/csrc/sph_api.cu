@@ -808,7 +808,7 @@ int allocate(sph_sim *s) {
 	    (rc = dalloc(&T.scenes, S)) || (rc = dalloc(&T.appCount, C)) || (rc = dalloc(&T.appStart, C)) ||
 	    (rc = dalloc(&T.appIdx, N)) || (rc = dalloc(&T.appCursor, C)) || (rc = dalloc(&T.newCell, N)) ||
 	    (rc = dalloc(&T.enterCount, C)) || (rc = dalloc(&T.leaveCount, C)) || (rc = dalloc(&T.enterOffset, C)) ||
-	    (rc = dalloc(&T.enterCursor, C)) || (rc = dalloc(&T.enterList, N)) || (rc = dalloc(&T.moverCount, 2)) ||
+	    (rc = dalloc(&T.enterCursor, C)) || (rc = dalloc(&T.enterList, N)) || (rc = dalloc(&T.moveMax, 1)) ||
 	    (rc = dalloc(&T.bbox, 4 * C)) || (rc = dalloc(&T.newIdx, N)) || (rc = dalloc(&T.newLabel, N)) ||
 	    (rc = dalloc(&T.taskCounter, 2)) || (rc = dalloc(&T.stats, 4 * S)) || (rc = dalloc(&T.error, 1)) ||
 	    (rc = dalloc(&T.scanTiles, 3 * ((C + kScanTile - 1) / kScanTile))) ||
@@ -826,7 +826,6 @@ int allocate(sph_sim *s) {
 	    (rc = dalloc(&s->doneV, std::max(C, appCap))) || (rc = dalloc(&T.refOrd, N)) ||
 	    (rc = dalloc(&T.viscBox, 4 * appCap)) || (rc = dalloc(&s->check, 4)))
 		return rc;
-	T.moverList = nullptr;
 	T.waitLimitNs = kDefaultWaitLimitNs;
 	T.hold[0] = T.hold[1] = -1;
 
@@ -1412,7 +1411,7 @@ int sph_destroy(sph_sim *s) {
 	void *ptrs[] = {s->cellStartA, s->cellCountA, s->cellStartB, s->cellCountB, T.taskOfCell,  T.taskCell,
 	                T.numberOrder, T.sceneOfCell, T.sceneOf,     T.scenes,      T.appScene,    T.appFrom,     T.appTo,
 	                T.appBox,      T.appCount,    T.appStart,    T.appIdx,      T.appCursor,   T.newCell,
-	                T.enterCount,  T.leaveCount,  T.enterOffset, T.enterCursor, T.enterList,   T.moverCount,
+	                T.enterCount,  T.leaveCount,  T.enterOffset, T.enterCursor, T.enterList,   T.moveMax,
 	                T.bbox,        T.newIdx,      T.newLabel,    T.taskCounter, T.stats,       T.error,
 	                T.scanTiles,   T.liveTask,    T.liveTiles,   T.nLive,
 	                T.abort,       T.bodies,      s->doneV,      s->doneD,      s->stagePos,   s->stageForce,

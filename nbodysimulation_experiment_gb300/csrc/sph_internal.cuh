@@ -142,7 +142,7 @@ struct SimTables {
 	int *appCount, *appStart, *appIdx, *appCursor;  // appendix members per cell
 	int *newCell;                      // cell after predict, per particle
 	int *enterCount, *leaveCount, *enterOffset, *enterCursor, *enterList;
-	int *moverList, *moverCount;       // moverCount[0]: movers; [1]: max cell move
+	int *moveMax;                      // longest cell move of the update
 	int *bbox;                         // per cell: x0, y0, x1, y1 of new cells
 	int *newCount, *newStart;
 	int *scanTiles;                    // 3 x tiles: per-tile sums, then tile offsets
