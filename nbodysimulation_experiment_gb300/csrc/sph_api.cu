@@ -597,8 +597,9 @@ int enqueue_step(sph_sim *s, bool capturing) {
 	bool anySprings = false;
 	for (const Scene &sc : s->scenes) anySprings = anySprings || sc.springs.enabled;
 	if (anySprings) {
-		k_springs_select<<<s->springBlocks, kSpringWarps * kWarp, springs_smem_bytes(), st>>>(tt, A.view(),
-		                                                                                      B.view(), T);
+		launch_springs_select(s->springBlocks, 2 * s->numSMs, st, tt, A.view(), B.view(), T);
+		SPH_LAUNCHED(s);
+		SPH_LAUNCHED(s);
 		SPH_LAUNCHED(s);
 		k_springs_commit<<<blocks_for(tt.n, kElemThreads), kElemThreads, 0, st>>>(tt, B.view(), T);
 		SPH_LAUNCHED(s);
@@ -809,6 +810,7 @@ int allocate(sph_sim *s) {
 	    (rc = dalloc(&T.appIdx, N)) || (rc = dalloc(&T.appCursor, C)) || (rc = dalloc(&T.newCell, N)) ||
 	    (rc = dalloc(&T.enterCount, C)) || (rc = dalloc(&T.leaveCount, C)) || (rc = dalloc(&T.enterOffset, C)) ||
 	    (rc = dalloc(&T.enterCursor, C)) || (rc = dalloc(&T.enterList, N)) || (rc = dalloc(&T.moveMax, 1)) ||
+	    (rc = dalloc(&T.springBig, 1)) ||
 	    (rc = dalloc(&T.bbox, 4 * C)) || (rc = dalloc(&T.newIdx, N)) || (rc = dalloc(&T.newLabel, N)) ||
 	    (rc = dalloc(&T.taskCounter, 2)) || (rc = dalloc(&T.stats, 4 * S)) || (rc = dalloc(&T.error, 1)) ||
 	    (rc = dalloc(&T.scanTiles, 3 * ((C + kScanTile - 1) / kScanTile))) ||
@@ -886,8 +888,7 @@ int allocate(sph_sim *s) {
 	if (sweep_attributes() != cudaSuccess ||
 	    cudaFuncSetAttribute(k_density, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dens_smem_bytes()) !=
 	        cudaSuccess ||
-	    cudaFuncSetAttribute(k_springs_select, cudaFuncAttributeMaxDynamicSharedMemorySize,
-	                         (int)springs_smem_bytes()) != cudaSuccess)
+	    !configure_springs_select())
 		return SPH_ERR_CUDA;
 	int occV = 0, occD = 0;
 	if (sweep_occupancy(false, kDeltaWide, &occV, &occD) != cudaSuccess || occV < 1 || occD < 1) return SPH_ERR_CUDA;
@@ -1411,7 +1412,7 @@ int sph_destroy(sph_sim *s) {
 	void *ptrs[] = {s->cellStartA, s->cellCountA, s->cellStartB, s->cellCountB, T.taskOfCell,  T.taskCell,
 	                T.numberOrder, T.sceneOfCell, T.sceneOf,     T.scenes,      T.appScene,    T.appFrom,     T.appTo,
 	                T.appBox,      T.appCount,    T.appStart,    T.appIdx,      T.appCursor,   T.newCell,
-	                T.enterCount,  T.leaveCount,  T.enterOffset, T.enterCursor, T.enterList,   T.moveMax,
+	                T.enterCount,  T.leaveCount,  T.enterOffset, T.enterCursor, T.enterList,   T.moveMax,     T.springBig,
 	                T.bbox,        T.newIdx,      T.newLabel,    T.taskCounter, T.stats,       T.error,
 	                T.scanTiles,   T.liveTask,    T.liveTiles,   T.nLive,
 	                T.abort,       T.bodies,      s->doneV,      s->doneD,      s->stagePos,   s->stageForce,

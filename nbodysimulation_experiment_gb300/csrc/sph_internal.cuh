@@ -143,6 +143,7 @@ struct SimTables {
 	int *newCell;                      // cell after predict, per particle
 	int *enterCount, *leaveCount, *enterOffset, *enterCursor, *enterList;
 	int *moveMax;                      // longest cell move of the update
+	int *springBig;                    // cells left to the larger spring stage (listed in enterList)
 	int *bbox;                         // per cell: x0, y0, x1, y1 of new cells
 	int *newCount, *newStart;
 	int *scanTiles;                    // 3 x tiles: per-tile sums, then tile offsets

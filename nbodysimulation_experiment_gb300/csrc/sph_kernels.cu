@@ -5,7 +5,7 @@
 //   k_viscosity     ordered viscosity sweep over the stale neighbour lists
 //                   (demo4.cpp:223-237, sph.h:497-512)
 //   k_predict       prev = x; x += v dt; new cell (demo4.cpp:329-347, sph.h:450-463)
-//   k_scan          prefix sums of the grid update
+//   k_scan_*        prefix sums of the grid update
 //   k_scatter       appendix and mover lists per cell
 //   k_grid_update   the reference's remove/insert grid update, event by event
 //                   (demo4.cpp:341-356, 37-76)
@@ -154,6 +154,7 @@ __global__ void k_integrate(Totals tt, Particles P, SimTables T, uint32_t *doneV
 	for (int k = i; k < nDoneD; k += threads) doneD[k] = 0u;
 	if (i == 0) {
 		*T.moveMax = 0;
+		*T.springBig = 0;
 		T.taskCounter[0] = 0;
 		T.taskCounter[1] = 0;
 	}
@@ -178,14 +179,14 @@ __global__ void k_integrate(Totals tt, Particles P, SimTables T, uint32_t *doneV
 // passed them once it is past slot own + k + 1.  So the head of k runs in
 // lockstep with the tail of k - 1 (its pairs after slot own + k), on the
 // other lane: the two touch disjoint slots.  The middle of k (its pairs with
-// k - 1, itself and k + 1) follows once k - 1 is finished, and k's tail runs
+// k - 1 and k + 1) follows once k - 1 is finished, and k's tail runs
 // beside the head of k + 1.  Each particle costs about the longer of its head
 // and tail instead of its whole list, with every pair in the reference's
 // order for each particle it touches.
 // This is the wide shape (ViscWide); the lean one, k_viscosity_multi below,
-// runs several tasks per block for throughput.  Both run the geometry inline
-// in the chain for particles with more in-range pairs than their geometry
-// buffer holds.
+// runs several tasks per block for throughput.  Particles with more in-range
+// pairs than their geometry buffer holds run the geometry inline in the chain
+// here; there they come in several segments.
 template <class C>
 struct ViscSmemT {
 	float2 pos[kStageCap];

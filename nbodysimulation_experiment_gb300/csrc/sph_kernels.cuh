@@ -119,7 +119,6 @@ inline int delta_stage_capacity(int shape) {
 void launch_viscosity(bool lean, int blocks, cudaStream_t st, Totals tt, Particles P, SimTables T);
 void launch_delta(int shape, int blocks, cudaStream_t st, Totals tt, Particles Q, SimTables T);
 size_t dens_smem_bytes();
-size_t springs_smem_bytes();
 
 __global__ void k_integrate(Totals tt, Particles P, SimTables T, uint32_t *doneV, int nDoneV, uint32_t *doneD,
                             int nDoneD);
@@ -150,7 +149,9 @@ __global__ void k_splat_points(int first, int count, const int *id, const float2
                                const float2 *press, const float2 *vel, float rho0, float halfW, float halfH,
                                float sx, float sy, int width, int height, unsigned long long *keys);
 __global__ void k_keys_to_rgba8(int pixels, const unsigned long long *keys, uint32_t *rgba);
-__global__ void k_springs_select(Totals tt, Particles P, Particles Q, SimTables T);
+void launch_springs_select(int blocks, int listedBlocks, cudaStream_t st, const Totals &tt, const Particles &P,
+                           const Particles &Q, const SimTables &T);
+bool configure_springs_select();
 __global__ void k_springs_commit(Totals tt, Particles Q, SimTables T);
 __global__ void k_springs_apply(Totals tt, Particles Q, SimTables T);
 __global__ void k_learned_z0(int n, int np, const float2 *pos, const float2 *prev, float invH, float2 *z0);

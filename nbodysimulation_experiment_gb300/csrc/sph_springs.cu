@@ -70,34 +70,45 @@ __device__ __forceinline__ int staged_index(int num, const int (&off)[9], const 
 // warp for one particle at a time (when at most kSpringWarpChoice of the 32
 // particles have free slots) or by every lane for its own particle with a
 // converged scan over the block.
+// Bound by dependent loads, so by the warps an SM holds, and these by shared
+// memory: with a stage of kStageCap entries a warp takes 26 KB, eight warps per
+// SM.  Most lists have fewer than 400 entries; a stage of 512 and 16-bit entry
+// numbers take 14 KB, sixteen warps (1M block 1,250 -> 770 us; 384 entries would
+// not let another block in).  Cells with longer lists are listed and run by a
+// second launch with the full stage (3 us when there are none).
 constexpr int kSpringWarpChoice = 16;
-struct SpringWarp {
-	float2 pos[kStageCap];
-	int tag[kStageCap];
+constexpr int kSpringStage = 512;
+template <int CAP>
+struct SpringWarpT {
+	float2 pos[CAP];
+	int tag[CAP];
 	// Per-lane lists, slot-major ([slot][lane]) so that the lanes' accesses
 	// fall on distinct banks.
-	int ex[kSprings][kWarp];     // existing partners (new numbers)
-	uint32_t exbits[kStageCap / 32][kWarp];  // per lane: staged entries that are existing partners
+	int16_t ex[kSprings][kWarp];  // existing partners (staged entries, or -1)
+	uint32_t exbits[CAP / 32][kWarp];  // per lane: staged entries that are existing partners
 	union {
 		struct {
 			float kr2[kSprings][kWarp];  // chosen candidates, sorted (per-lane scan)
 			int ktag[kSprings][kWarp];
-			int kj[kSprings][kWarp];
+			int16_t kj[kSprings][kWarp];  // staged entries
 		};
-		unsigned long long key[kStageCap];  // one particle's candidate keys (warp-wide choice)
+		unsigned long long key[CAP];  // one particle's candidate keys (warp-wide choice)
 	};
 };
 
-size_t springs_smem_bytes() { return sizeof(SpringWarp) * kSpringWarps; }
 
+template <int CAP, bool kListed>
 __global__ void __launch_bounds__(kSpringWarps * kWarp) k_springs_select(Totals tt, Particles P, Particles Q,
                                                                         SimTables T) {
+	using SpringWarp = SpringWarpT<CAP>;
 	extern __shared__ __align__(16) unsigned char smem_raw[];
 	SpringWarp &S = reinterpret_cast<SpringWarp *>(smem_raw)[threadIdx.x / kWarp];
 	const int lane = threadIdx.x & (kWarp - 1);
-	for (int w = 0; w < kStageCap / 32; ++w) S.exbits[w][lane] = 0u;
+	for (int w = 0; w < CAP / 32; ++w) S.exbits[w][lane] = 0u;
 	const int warpsTotal = gridDim.x * kSpringWarps;
-	for (int c = blockIdx.x * kSpringWarps + threadIdx.x / kWarp; c < tt.ncell; c += warpsTotal) {
+	const int items = kListed ? *T.springBig : tt.ncell;
+	for (int w = blockIdx.x * kSpringWarps + threadIdx.x / kWarp; w < items; w += warpsTotal) {
+		const int c = kListed ? T.enterList[w] : w;
 		const int cnt = T.newCount[c];
 		if (cnt == 0) continue;
 		const SceneDev &sc = T.scenes[T.sceneOfCell[c]];
@@ -122,6 +133,10 @@ __global__ void __launch_bounds__(kSpringWarps * kWarp) k_springs_select(Totals 
 		}
 		if (L > kStageCap) {
 			if (lane == 0) atomicOr(T.error, kErrStageOverflow);
+			continue;
+		}
+		if (L > CAP) {
+			if (lane == 0) T.enterList[atomicAdd(T.springBig, 1)] = c;
 			continue;
 		}
 		for (int e = lane; e < L; e += kWarp) {
@@ -175,7 +190,7 @@ __global__ void __launch_bounds__(kSpringWarps * kWarp) k_springs_select(Totals 
 					if (q >= ne) break;
 					float rest = rl[q];
 					const int e = staged_index(pn[q], segOff, segStart, L);
-					S.ex[q][lane] = e;
+					S.ex[q][lane] = (int16_t)e;
 					if (e >= 0) S.exbits[e >> 5][lane] |= 1u << (e & 31);
 					const float2 xp = e >= 0 ? S.pos[e] : Q.pos[pn[q]];
 					const float rx = xp.x - xi.x, ry = xp.y - xi.y;
@@ -259,12 +274,12 @@ __global__ void __launch_bounds__(kSpringWarps * kWarp) k_springs_select(Totals 
 				}
 				S.kr2[at][lane] = r2;
 				S.ktag[at][lane] = tj;
-				S.kj[at][lane] = num;
+				S.kj[at][lane] = (int16_t)e;
 			}
 			if (active) {
 				T.accN[j] = kc;
 				if (perLane)
-					for (int q = 0; q < kc; ++q) T.accP[j * kSprings + q] = S.kj[q][lane];
+					for (int q = 0; q < kc; ++q) T.accP[j * kSprings + q] = seg_number<9>(S.kj[q][lane], segOff, segStart);
 				Q.springN[j] = m;
 				for (int q = 0; q < ne; ++q) {
 					const int e = S.ex[q][lane];
@@ -275,6 +290,21 @@ __global__ void __launch_bounds__(kSpringWarps * kWarp) k_springs_select(Totals 
 		}
 		__syncwarp();
 	}
+}
+
+void launch_springs_select(int blocks, int listedBlocks, cudaStream_t st, const Totals &tt, const Particles &P,
+                           const Particles &Q, const SimTables &T) {
+	k_springs_select<kSpringStage, false>
+	    <<<blocks, kSpringWarps * kWarp, sizeof(SpringWarpT<kSpringStage>) * kSpringWarps, st>>>(tt, P, Q, T);
+	k_springs_select<kStageCap, true>
+	    <<<listedBlocks, kSpringWarps * kWarp, sizeof(SpringWarpT<kStageCap>) * kSpringWarps, st>>>(tt, P, Q, T);
+}
+
+bool configure_springs_select() {
+	return cudaFuncSetAttribute(k_springs_select<kSpringStage, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+	                            (int)(sizeof(SpringWarpT<kSpringStage>) * kSpringWarps)) == cudaSuccess &&
+	       cudaFuncSetAttribute(k_springs_select<kStageCap, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+	                            (int)(sizeof(SpringWarpT<kStageCap>) * kSpringWarps)) == cudaSuccess;
 }
 
 // A spring joins both ends where each chose the other.
