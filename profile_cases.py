@@ -72,7 +72,7 @@ def batched(updates: int = 3) -> None:
     batch = BatchSimulation(mix)
     batch.update(float(scenes.DT))
     sms = batch.sweep_shape()[1] // 4  # the default viscosity shape runs 4 blocks per SM
-    batch.set_sweep_shape((VISC_WARPS[1], 3 * sms, DELTA_WARPS[1], 8 * sms))
+    batch.set_sweep_shape((VISC_WARPS[1], sms, DELTA_WARPS[1], 8 * sms))
     for _ in range(updates):
         batch.update(float(scenes.DT))
     batch.synchronize()
@@ -117,8 +117,8 @@ def learned_dam(frames: int = 3) -> None:
 def block(side: int = 512, updates: int = 3) -> None:
     """A side x side jittered block with springs on (yield 0.1, plasticity
     0.3, stiffness 0.3, at most 16), in the sweep shapes the autotuner picks
-    for the 1,048,576-particle block (lean 5-warp viscosity at 3 blocks per
-    SM, pipelined 3-warp delta at 5 per SM): 3 + `updates` updates."""
+    for the 1,048,576-particle block (lean viscosity at one block per SM,
+    pipelined 3-warp delta at 5 per SM): 3 + `updates` updates."""
     scene = scenes.block_1m() if side == 1024 else scenes.scaled_block(side, seed=3, obstacles=False)
     sim = Simulation(scene.domain())
     scene.apply(sim)
@@ -126,7 +126,7 @@ def block(side: int = 512, updates: int = 3) -> None:
     for _ in range(3):
         sim.update(float(scenes.DT))
     sms = sim.sweep_shape()[3]  # the default delta shape runs one block per SM
-    sim.set_sweep_shape((VISC_WARPS[1], 3 * sms, DELTA_WARPS[3], 5 * sms))
+    sim.set_sweep_shape((VISC_WARPS[1], sms, DELTA_WARPS[3], 5 * sms))
     for _ in range(updates):
         sim.update(float(scenes.DT))
     sim.synchronize()
