@@ -597,9 +597,9 @@ int enqueue_step(sph_sim *s, bool capturing) {
 	bool anySprings = false;
 	for (const Scene &sc : s->scenes) anySprings = anySprings || sc.springs.enabled;
 	if (anySprings) {
-		launch_springs_select(s->springBlocks, 2 * s->numSMs, st, tt, A.view(), B.view(), T);
+		launch_springs_select(s->springBlocks, st, tt, A.view(), B.view(), T);
 		SPH_LAUNCHED(s);
-		SPH_LAUNCHED(s);
+		launch_springs_select_listed(2 * s->numSMs, st, tt, A.view(), B.view(), T);
 		SPH_LAUNCHED(s);
 		k_springs_commit<<<blocks_for(tt.n, kElemThreads), kElemThreads, 0, st>>>(tt, B.view(), T);
 		SPH_LAUNCHED(s);

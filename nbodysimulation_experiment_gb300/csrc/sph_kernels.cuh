@@ -149,8 +149,10 @@ __global__ void k_splat_points(int first, int count, const int *id, const float2
                                const float2 *press, const float2 *vel, float rho0, float halfW, float halfH,
                                float sx, float sy, int width, int height, unsigned long long *keys);
 __global__ void k_keys_to_rgba8(int pixels, const unsigned long long *keys, uint32_t *rgba);
-void launch_springs_select(int blocks, int listedBlocks, cudaStream_t st, const Totals &tt, const Particles &P,
-                           const Particles &Q, const SimTables &T);
+void launch_springs_select(int blocks, cudaStream_t st, const Totals &tt, const Particles &P, const Particles &Q,
+                           const SimTables &T);
+void launch_springs_select_listed(int blocks, cudaStream_t st, const Totals &tt, const Particles &P,
+                                  const Particles &Q, const SimTables &T);
 bool configure_springs_select();
 __global__ void k_springs_commit(Totals tt, Particles Q, SimTables T);
 __global__ void k_springs_apply(Totals tt, Particles Q, SimTables T);

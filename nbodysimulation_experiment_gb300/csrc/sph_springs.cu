@@ -292,12 +292,17 @@ __global__ void __launch_bounds__(kSpringWarps * kWarp) k_springs_select(Totals 
 	}
 }
 
-void launch_springs_select(int blocks, int listedBlocks, cudaStream_t st, const Totals &tt, const Particles &P,
-                           const Particles &Q, const SimTables &T) {
+void launch_springs_select(int blocks, cudaStream_t st, const Totals &tt, const Particles &P, const Particles &Q,
+                           const SimTables &T) {
 	k_springs_select<kSpringStage, false>
 	    <<<blocks, kSpringWarps * kWarp, sizeof(SpringWarpT<kSpringStage>) * kSpringWarps, st>>>(tt, P, Q, T);
+}
+
+// The cells that the first launch left in the list.
+void launch_springs_select_listed(int blocks, cudaStream_t st, const Totals &tt, const Particles &P,
+                                  const Particles &Q, const SimTables &T) {
 	k_springs_select<kStageCap, true>
-	    <<<listedBlocks, kSpringWarps * kWarp, sizeof(SpringWarpT<kStageCap>) * kSpringWarps, st>>>(tt, P, Q, T);
+	    <<<blocks, kSpringWarps * kWarp, sizeof(SpringWarpT<kStageCap>) * kSpringWarps, st>>>(tt, P, Q, T);
 }
 
 bool configure_springs_select() {
