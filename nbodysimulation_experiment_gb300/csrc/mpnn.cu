@@ -83,6 +83,7 @@ struct sph_mpnn {
 	float2 *z[kRounds + 1] = {};  // z[0] unused (the graph's z0)
 	float2 *dz[kRounds + 1] = {};
 	float2 *dzEdge = nullptr, *u = nullptr;
+	float *sums = nullptr;  // kReduceParts x kRounds x kSumsRow
 	__nv_bfloat16 *da3b = nullptr, *da3f = nullptr, *dXb = nullptr, *dXf = nullptr;
 	float *dX = nullptr, *dH = nullptr;
 	float *loss = nullptr;
@@ -192,13 +193,14 @@ int backward(sph_mpnn *m, const MpnnGraph &G, const float2 *target, cudaStream_t
 	for (int r = kRounds - 1; r >= 0; --r) {
 		const float *P = m->params + (size_t)r * kRoundParams;
 		float *Gp = m->grads + (size_t)r * kRoundParams;
+		float *sums = m->sums + r * kSumsRow;
 		const float2 *zr = r == 0 ? G.z0 : m->z[r];
 		k_mpnn_node_bwd<<<blocks((size_t)np * kWarp, 256), 256, 0, st>>>(dzNext, P + kOffW4, m->cb[r], m->da3b, np);
 		MPNN_CUDA(cudaGetLastError());
 		dim3 tg(blocks(kHidden, 32), blocks(np, 32));
 		k_mpnn_transpose<<<tg, dim3(32, 8), 0, st>>>(m->da3b, np, kHidden, kHidden, m->da3f, np);
-		k_mpnn_dw4<<<dim3(kHidden, kReduceParts), kReduceThreads, 0, st>>>(dzNext, m->cf[r], np, n, Gp + kOffW4, Gp + kOffB4);
-		k_mpnn_rowsum<<<dim3(kHidden, kReduceParts), kReduceThreads, 0, st>>>(m->da3f, np, n, nullptr, Gp + kOffB3);
+		k_mpnn_dw4<<<dim3(kHidden, kReduceParts), kReduceThreads, 0, st>>>(dzNext, m->cf[r], np, n, sums);
+		k_mpnn_rowsum<<<dim3(kHidden, kReduceParts), kReduceThreads, 0, st>>>(m->da3f, np, n, nullptr, sums + kSumsB3);
 		MPNN_CUDA(cudaGetLastError());
 		// dW3 += da3^T X3 (reduction over particles).
 		GemmArgs g3 = gemm(m->da3f, np, m->X3f[r], np, kHidden, kNodeInPad, np, m->error);
@@ -218,7 +220,7 @@ int backward(sph_mpnn *m, const MpnnGraph &G, const float2 *target, cudaStream_t
 		g4.ldcbT = np;
 		rc = run_gemm(g4, 1, st);
 		if (rc) return rc;
-		k_mpnn_rowsum<<<dim3(kHidden, kReduceParts), kReduceThreads, 0, st>>>(m->dXf, np, n, m->degS, Gp + kOffB2);
+		k_mpnn_rowsum<<<dim3(kHidden, kReduceParts), kReduceThreads, 0, st>>>(m->dXf, np, n, m->degS, sums + kSumsB2);
 		MPNN_CUDA(cudaGetLastError());
 		// dW2 += dM^T H.
 		GemmArgs g5 = gemm(m->dXf, np, m->Hf[r], np, kHidden, kHidden, np, m->error);
@@ -246,6 +248,8 @@ int backward(sph_mpnn *m, const MpnnGraph &G, const float2 *target, cudaStream_t
 			dzNext = m->dz[r];
 		}
 	}
+	k_mpnn_add_sums<<<blocks(kRounds * kSumsRow, 128), 128, 0, st>>>(m->sums, m->grads);
+	MPNN_CUDA(cudaGetLastError());
 	return SPH_OK;
 }
 
@@ -332,7 +336,7 @@ int sph_mpnn_destroy(sph_mpnn *m) {
 	for (Sample &s : m->samples) s.release();
 	std::vector<void *> ptrs = {m->params, m->grads, m->adamM, m->adamV, m->W2b, m->W2Tb, m->W3b, m->W3Tb,
 	                            m->degS,   m->dzEdge, m->u,    m->da3b,  m->da3f, m->dXb, m->dXf, m->dX,
-	                            m->dH,     m->loss,  m->error};
+	                            m->dH,     m->sums,  m->loss, m->error};
 	for (int r = 0; r < kRounds; ++r) {
 		ptrs.insert(ptrs.end(), {m->Hb[r], m->Hf[r], m->X3b[r], m->X3f[r], m->cb[r], m->cf[r]});
 	}
@@ -377,7 +381,8 @@ int sph_mpnn_create(int device, size_t max_particles, uint64_t seed, sph_mpnn **
 	    (rc = zalloc(&m->dzEdge, C)) || (rc = zalloc(&m->u, C)) || (rc = zalloc(&m->da3b, C * kHidden)) ||
 	    (rc = zalloc(&m->da3f, C * kHidden)) || (rc = zalloc(&m->dXb, C * kNodeInPad)) ||
 	    (rc = zalloc(&m->dXf, C * kNodeInPad)) || (rc = zalloc(&m->dX, C * kNodeInPad)) ||
-	    (rc = zalloc(&m->dH, C * kHidden)) || (rc = zalloc(&m->loss, 1)) || (rc = zalloc(&m->error, 1)))
+	    (rc = zalloc(&m->dH, C * kHidden)) || (rc = zalloc(&m->sums, kReduceParts * kRounds * kSumsRow)) ||
+	    (rc = zalloc(&m->loss, 1)) || (rc = zalloc(&m->error, 1)))
 		return fail(rc);
 	for (int r = 0; r < kRounds; ++r) {
 		if ((rc = zalloc(&m->Hb[r], C * kHidden)) || (rc = zalloc(&m->Hf[r], C * kHidden)) ||

@@ -83,6 +83,10 @@ constexpr int kEdgeWarps = 4;
 constexpr int kBwdWarps = 8;        // k_mpnn_edge_bwd: warps sharing a cell's staged block
 constexpr int kReduceThreads = 256;  // row sums over the particles
 constexpr int kReduceParts = 8;      // blocks per row
+// Their sums, per part and round: b2, b3, W4, b4.
+constexpr int kSumsB2 = 0, kSumsB3 = kSumsB2 + kHidden, kSumsW4 = kSumsB3 + kHidden,
+              kSumsRow = kSumsW4 + 2 * kHidden + 2;
+static_assert(kOffW4 - kOffB3 == kSumsW4 - kSumsB3 && kRoundParams - kOffB3 == kSumsRow - kSumsB3, "same order");
 size_t mpnn_edge_smem(bool backward);
 size_t mpnn_edge_tc_smem();
 int mpnn_edge_tc_blocks_per_sm();
@@ -101,8 +105,9 @@ __global__ void k_mpnn_loss(const float2 *z2, const float2 *z0, const float2 *ta
                             float *loss);
 __global__ void k_mpnn_node_bwd(const float2 *dz, const float *W4, const __nv_bfloat16 *cb, __nv_bfloat16 *da3b,
                                 int np);
-__global__ void k_mpnn_dw4(const float2 *dz, const __nv_bfloat16 *cf, int ldf, int n, float *gW4, float *gb4);
-__global__ void k_mpnn_rowsum(const __nv_bfloat16 *X, int ld, int n, const float *w, float *out);
+__global__ void k_mpnn_dw4(const float2 *dz, const __nv_bfloat16 *cf, int ldf, int n, float *sums);
+__global__ void k_mpnn_rowsum(const __nv_bfloat16 *X, int ld, int n, const float *w, float *sums);
+__global__ void k_mpnn_add_sums(const float *sums, float *grads);
 __global__ void k_mpnn_combine(const float2 *dzNext, const float *dX, const float2 *dzEdge, float2 *dz, int n,
                                int np);
 __global__ void k_mpnn_transpose(const __nv_bfloat16 *src, int rows, int cols, int lds, __nv_bfloat16 *dst, int ldd);

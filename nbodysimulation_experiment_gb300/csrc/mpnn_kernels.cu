@@ -740,7 +740,11 @@ __global__ void k_mpnn_node_bwd(const float2 *dz, const float *W4, const __nv_bf
 
 // Sums over the particles of a feature-major row: kReduceParts blocks a row,
 // eight values a load.  (One block a row and one value a load: 117 us for 128
-// rows of 65,536, which are 17 MB; 8 us now, k_mpnn_dw4 118 and 20.)
+// rows of 65,536, which are 17 MB; 8 us now, k_mpnn_dw4 118 and 20.)  The
+// blocks' sums go to `sums` (kSumsRow values a part and round) and are added in
+// the order of the parts by k_mpnn_add_sums (2.6 us a gradient), so they repeat
+// bit for bit; with an atomic from each block they did not.  (The parts as a cluster that adds
+// in distributed shared memory: 8 blocks 28 and 10 us, 4 blocks 22 and 11.)
 namespace {
 
 template <class F>
@@ -761,8 +765,8 @@ __device__ __forceinline__ void reduce_row(const __nv_bfloat16 *row, int n, F f)
 	}
 }
 
-// *out += the block's sum of v.
-__device__ __forceinline__ void block_add(float v, float *out) {
+// *out = the block's sum of v.
+__device__ __forceinline__ void block_sum(float v, float *out) {
 	__shared__ float part[kReduceThreads / kWarp];
 	v = warp_sum(v);
 	if ((threadIdx.x & (kWarp - 1)) == 0) part[threadIdx.x / kWarp] = v;
@@ -770,18 +774,19 @@ __device__ __forceinline__ void block_add(float v, float *out) {
 	if (threadIdx.x == 0) {
 		float s = 0.f;
 		for (int w = 0; w < kReduceThreads / kWarp; ++w) s += part[w];
-		atomicAdd(out, s);
+		*out = s;
 	}
 	__syncthreads();
 }
 
 }  // namespace
 
-// gW4[o][f] += sum_i dz_i[o] c_i[f], f = blockIdx.x (one per hidden feature);
-// f = 0 also adds gb4 += sum_i dz_i.
+// W4's sums, sum_i dz_i[o] c_i[f], f = blockIdx.x (one per hidden feature);
+// f = 0 also takes b4's, sum_i dz_i.
 __global__ void __launch_bounds__(kReduceThreads) k_mpnn_dw4(const float2 *dz, const __nv_bfloat16 *cf, int ldf, int n,
-                                                              float *gW4, float *gb4) {
+                                                              float *sums) {
 	const int f = blockIdx.x;
+	float *out = sums + blockIdx.y * kRounds * kSumsRow + kSumsW4;
 	float a0 = 0.f, a1 = 0.f, s0 = 0.f, s1 = 0.f;
 	reduce_row(cf + (size_t)f * ldf, n, [&](int i, float c) {
 		const float2 g = dz[i];
@@ -790,20 +795,31 @@ __global__ void __launch_bounds__(kReduceThreads) k_mpnn_dw4(const float2 *dz, c
 		s0 += g.x;
 		s1 += g.y;
 	});
-	block_add(a0, gW4 + f);
-	block_add(a1, gW4 + kHidden + f);
+	block_sum(a0, out + f);
+	block_sum(a1, out + kHidden + f);
 	if (f == 0) {
-		block_add(s0, gb4);
-		block_add(s1, gb4 + 1);
+		block_sum(s0, out + 2 * kHidden);
+		block_sum(s1, out + 2 * kHidden + 1);
 	}
 }
 
-// out[r] += sum_{i<n} X[r][i] (* w[i]); row blockIdx.x, part blockIdx.y.
+// sum_{i<n} X[r][i] (* w[i]); row r = blockIdx.x, part blockIdx.y.
 __global__ void __launch_bounds__(kReduceThreads) k_mpnn_rowsum(const __nv_bfloat16 *X, int ld, int n, const float *w,
-                                                                 float *out) {
+                                                                 float *sums) {
 	float s = 0.f;
 	reduce_row(X + (size_t)blockIdx.x * ld, n, [&](int i, float x) { s += w ? x * w[i] : x; });
-	block_add(s, out + blockIdx.x);
+	block_sum(s, sums + blockIdx.y * kRounds * kSumsRow + blockIdx.x);
+}
+
+// The gradients of b2, b3, W4 and b4 of every round from the parts' sums.
+__global__ void k_mpnn_add_sums(const float *sums, float *grads) {
+	const int i = blockIdx.x * blockDim.x + threadIdx.x;
+	if (i >= kRounds * kSumsRow) return;
+	float s = 0.f;
+	for (int p = 0; p < kReduceParts; ++p) s += sums[p * kRounds * kSumsRow + i];
+	const int r = i / kSumsRow, k = i % kSumsRow;
+	// b3, W4 and b4 follow one another in both layouts.
+	grads[r * kRoundParams + (k < kSumsB3 ? kOffB2 + k : kOffB3 + (k - kSumsB3))] = s;
 }
 
 // dz_r = dz_{r+1} + (dX3 columns of z) + edge term, zero on the padding.
