@@ -550,6 +550,10 @@ int enqueue_step(sph_sim *s, bool capturing) {
 			k_live_reduce<<<ntiles, kScanThreads, 0, st>>>(tt, T);
 			SPH_LAUNCHED(s);
 		}
+		if (ntiles > kScanFewTiles) {
+			k_tile_offsets<<<1, kScanThreads, 0, st>>>(T.liveTiles, ntiles);
+			SPH_LAUNCHED(s);
+		}
 		k_live_apply<<<ntiles, kScanThreads, 0, st>>>(tt, T);
 		SPH_LAUNCHED(s);
 	}
@@ -583,6 +587,10 @@ int enqueue_step(sph_sim *s, bool capturing) {
 		const int ntiles = (tt.ncell + kScanTile - 1) / kScanTile;
 		if (ntiles > 1) {
 			k_scan_reduce<<<ntiles, kScanThreads, 0, st>>>(tt, T);
+			SPH_LAUNCHED(s);
+		}
+		if (ntiles > kScanFewTiles) {
+			k_tile_offsets<<<3, kScanThreads, 0, st>>>(T.scanTiles, ntiles);
 			SPH_LAUNCHED(s);
 		}
 		k_scan_apply<<<ntiles, kScanThreads, 0, st>>>(tt, T);

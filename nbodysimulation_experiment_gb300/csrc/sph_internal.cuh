@@ -146,8 +146,8 @@ struct SimTables {
 	int *springBig;                    // cells left to the larger spring stage (listed in enterList)
 	int *bbox;                         // per cell: x0, y0, x1, y1 of new cells
 	int *newCount, *newStart;
-	int *scanTiles;                    // 3 x tiles: per-tile sums
-	int *liveTask, *liveTiles, *nLive;  // occupied canonical cells' tasks in order, per-tile counts, count
+	int *scanTiles;                    // 3 x tiles: per-tile sums (or offsets, k_tile_offsets)
+	int *liveTask, *liveTiles, *nLive;  // occupied canonical cells' tasks in order, per-tile counts (or offsets), count
 	int *newIdx;    // new number -> old number (the new cell arrays, concatenated)
 	int *newLabel;  // old number -> new number
 	uint32_t *done;                    // per sweep task

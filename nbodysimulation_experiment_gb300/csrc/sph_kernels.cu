@@ -1268,55 +1268,109 @@ __device__ __forceinline__ void load_four(int (&v)[4], const int *p, int r, int 
 	}
 }
 
-// Block-wide exclusive scans of N values per thread (kScanThreads threads),
-// each on top of the sums of the `tile` tiles before this one, whose sums lie
-// at tiles[q * ntiles].  v[q] becomes the prefix; the thread of warp q's last
-// lane returns the sum up to and including this tile, others 0.  One use of
-// warpSums per kernel.
-template <int N>
-__device__ __forceinline__ int block_exscan(int (&v)[N], int (*warpSums)[kWarp], const int *tiles, int tile,
+// The running prefix from `first` over four consecutive values into a table's
+// positions from r on.
+__device__ __forceinline__ void store_prefix(int *p, int r, int n, int first, const int (&v)[4]) {
+	const int4 x = make_int4(first, first + v[0], first + v[0] + v[1], first + v[0] + v[1] + v[2]);
+	if (r + 4 <= n) {
+		*reinterpret_cast<int4 *>(p + r) = x;
+	} else {
+		if (r < n) p[r] = x.x;
+		if (r + 1 < n) p[r + 1] = x.y;
+		if (r + 2 < n) p[r + 2] = x.z;
+	}
+}
+
+// Block-wide exclusive scans (kScanThreads threads) of N tables, each on top of
+// the `tile` tiles before this one: tiles[q * ntiles] holds the tiles' sums or,
+// past kScanFewTiles of them, their offsets.  A thread brings one value of each
+// table, of the last one a value of each of S consecutive parts of the tile.
+// v[q] becomes the prefix; the thread of warp q's last lane returns the sum up
+// to and including this tile, or this part, others 0.  One use of sums per
+// kernel.
+template <int N, int S>
+__device__ __forceinline__ int block_exscan(int (&v)[N - 1 + S], int (*sums)[kWarp], const int *tiles, int tile,
                                             int ntiles) {
-	static_assert(kScanThreads == kWarp * kWarp && N <= kWarp, "one value per lane of the second level");
+	constexpr int V = N - 1 + S;
+	static_assert(kScanThreads == kWarp * kWarp && V <= kWarp, "one value per lane of the second level");
 	const int lane = threadIdx.x & (kWarp - 1), warp = threadIdx.x / kWarp;
-	int incl[N];
+	int incl[V];
 #pragma unroll
-	for (int q = 0; q < N; ++q) {
+	for (int q = 0; q < V; ++q) {
 		incl[q] = v[q];
 #pragma unroll
 		for (int o = 1; o < kWarp; o <<= 1) {
 			const int t = __shfl_up_sync(kFull, incl[q], o);
 			if (lane >= o) incl[q] += t;
 		}
-		if (lane == kWarp - 1) warpSums[q][warp] = incl[q];
+		if (lane == kWarp - 1) sums[q][warp] = incl[q];
 	}
 	int before = 0, total = 0;
-	if (warp < N) {
+	if (warp < N && ntiles > kScanFewTiles) {
+		before = tiles[warp * ntiles + tile];
+	} else if (warp < N) {
 		for (int i = lane; i < tile; i += kWarp) before += tiles[warp * ntiles + i];
 #pragma unroll
 		for (int o = 16; o > 0; o >>= 1) before += __shfl_xor_sync(kFull, before, o);
 	}
 	__syncthreads();
-	if (warp < N) {
-		const int w = warpSums[warp][lane];
+	if (warp < V) {
+		const int w = sums[warp][lane];
 		int wi = w;
 #pragma unroll
 		for (int o = 1; o < kWarp; o <<= 1) {
 			const int t = __shfl_up_sync(kFull, wi, o);
 			if (lane >= o) wi += t;
 		}
-		warpSums[warp][lane] = before + wi - w;
-		if (lane == kWarp - 1) total = before + wi;
+		sums[warp][lane] = before + wi - w;
+		if (lane == kWarp - 1) sums[V][warp] = total = before + wi;
 	}
 	__syncthreads();
+	int part = 0;  // sum of the parts before (the first one's includes the tiles before)
 #pragma unroll
-	for (int q = 0; q < N; ++q) v[q] = warpSums[q][warp] + incl[q] - v[q];
+	for (int q = 0; q < V; ++q) {
+		v[q] = sums[q][warp] + incl[q] - v[q] + part;
+		if (q >= N - 1) part += sums[V][q];
+	}
 	return total;
 }
 
 }  // namespace
 
+// The sums of ntiles tiles at tiles[blockIdx.x * ntiles] become the tiles'
+// offsets.  For grids of more than kScanFewTiles tiles: there each block of the
+// next pass would add up the sums before its own, a time that grows with the
+// number of tiles for each of them (both passes of an update on 2^26 cells,
+// 16,382 tiles: 2.25 ms more than with this pass; equal at 512 tiles, 3 us
+// less without it at 64).
+__global__ void __launch_bounds__(kScanThreads) k_tile_offsets(int *tiles, int ntiles) {
+	__shared__ int sums[2][kWarp], carry;
+	int *row = tiles + (size_t)blockIdx.x * ntiles;
+	int before = 0;
+	for (int base = 0; base < ntiles; base += 4 * kScanThreads) {
+		int x[4], v[1] = {0};
+		const int r = base + 4 * threadIdx.x;
+#pragma unroll
+		for (int k = 0; k < 4; ++k) {
+			x[k] = r + k < ntiles ? row[r + k] : 0;
+			v[0] += x[k];
+		}
+		const int total = block_exscan<1, 1>(v, sums, nullptr, 0, 1);
+		if (threadIdx.x == kWarp - 1) carry = total;
+		v[0] += before;
+#pragma unroll
+		for (int k = 0; k < 4; ++k) {
+			if (r + k < ntiles) row[r + k] = v[0];
+			v[0] += x[k];
+		}
+		__syncthreads();
+		before += carry;
+		__syncthreads();
+	}
+}
+
 __global__ void __launch_bounds__(kScanThreads) k_live_apply(Totals tt, SimTables T) {
-	__shared__ int warpSums[1][kWarp];
+	__shared__ int sums[2][kWarp];
 	const int tile = blockIdx.x, r = tile * kScanTile + 4 * threadIdx.x;
 	int c[4], v[1] = {0};
 	bool live[4];
@@ -1326,7 +1380,7 @@ __global__ void __launch_bounds__(kScanThreads) k_live_apply(Totals tt, SimTable
 		live[k] = r + k < tt.ncell && T.cellCount[c[k]] > 0;
 		v[0] += live[k];
 	}
-	const int total = block_exscan(v, warpSums, T.liveTiles, tile, gridDim.x);
+	const int total = block_exscan<1, 1>(v, sums, T.liveTiles, tile, gridDim.x);
 	if (tile == gridDim.x - 1 && threadIdx.x == kWarp - 1) *T.nLive = total;
 #pragma unroll
 	for (int k = 0; k < 4; ++k)
@@ -1336,13 +1390,18 @@ __global__ void __launch_bounds__(kScanThreads) k_live_apply(Totals tt, SimTable
 // ---------------------------------------------------------------------------
 // Exclusive scans over cells, in two passes over tiles of kScanTile positions:
 // per-tile sums (not launched for a single tile), then per-tile scans, each
-// block adding up the sums of the tiles before its own.  Three scans run
+// block adding up the sums of the tiles before its own, or past kScanFewTiles
+// reading them from a pass between (k_tile_offsets).  Three scans run
 // together: the appendix counts and the entering counts in cell order, and
 // the new cell counts (cellCount + appCount - leaveCount + enterCount) in
 // numbering order (scenes in order, cells in colour rank).  Bound by launches
-// and barriers, not by the few bytes: a thread takes four consecutive
-// positions, so a block has two barriers (36 with one position at a time and
-// one scan after another) and no launch is needed for the tile sums.
+// and barriers on small grids, not by the few bytes: all values of a tile are
+// scanned at once, so a block has two barriers (36 with one position at a time
+// and one scan after another).  On large ones by the accesses by cell of the
+// new counts: a thread takes one position in each quarter of the tile for
+// them, so that a warp's are near one another, and four consecutive positions
+// of the two tables in cell order (four consecutive ones of all three: 102
+// against 60 us on 2048 x 2048 cells, 9.8 against 8.4 on 512 x 512).
 // Together with the task list above and the task flags cleared in k_integrate
 // instead of by four memsets: 451 -> 425 us per update at 256 particles,
 // 1,527 -> 1,503 at 4,096 (dam break), 2,836 -> 2,816 at 65,536.
@@ -1392,31 +1451,30 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_reduce(Totals tt, SimTabl
 // newCount and newStart.  Also restarts the per-scene neighbour-count
 // statistics (demo4.cpp:369-370).
 __global__ void __launch_bounds__(kScanThreads) k_scan_apply(Totals tt, SimTables T) {
-	__shared__ int warpSums[3][kWarp];
-	const int t = blockIdx.x, r = t * kScanTile + 4 * threadIdx.x;
-	int a[4], e[4], c[4], nw[4], v[3] = {0, 0, 0};
+	constexpr int kParts = kScanTile / kScanThreads;
+	static_assert(kParts == 4, "load_four");
+	__shared__ int sums[3 + kParts][kWarp];
+	const int t = blockIdx.x, r = t * kScanTile + 4 * threadIdx.x, r0 = t * kScanTile + threadIdx.x;
+	int a[4], e[4], c[kParts], nw[kParts], v[2 + kParts] = {};
 	load_four(a, T.appCount, r, tt.ncell);
 	load_four(e, T.enterCount, r, tt.ncell);
-	load_four(c, T.numberOrder, r, tt.ncell);
 #pragma unroll
-	for (int k = 0; k < 4; ++k) {
-		nw[k] = r + k < tt.ncell ? new_count(T, c[k]) : 0;
+	for (int k = 0; k < kParts; ++k) {
+		const int p = r0 + k * kScanThreads;
+		c[k] = p < tt.ncell ? T.numberOrder[p] : -1;
+		nw[k] = v[2 + k] = c[k] >= 0 ? new_count(T, c[k]) : 0;
 		v[0] += a[k];
 		v[1] += e[k];
-		v[2] += nw[k];
 	}
-	block_exscan(v, warpSums, T.scanTiles, t, gridDim.x);
+	block_exscan<3, kParts>(v, sums, T.scanTiles, t, gridDim.x);
+	store_prefix(T.appStart, r, tt.ncell, v[0], a);
+	store_prefix(T.enterOffset, r, tt.ncell, v[1], e);
 #pragma unroll
-	for (int k = 0; k < 4; ++k) {
-		if (r + k < tt.ncell) {
-			T.appStart[r + k] = v[0];
-			T.enterOffset[r + k] = v[1];
+	for (int k = 0; k < kParts; ++k) {
+		if (c[k] >= 0) {
 			T.newCount[c[k]] = nw[k];
-			T.newStart[c[k]] = v[2];
+			T.newStart[c[k]] = v[2 + k];
 		}
-		v[0] += a[k];
-		v[1] += e[k];
-		v[2] += nw[k];
 	}
 	if (t == 0) {
 		for (int sc = threadIdx.x; sc < tt.nscenes; sc += blockDim.x) {

@@ -97,6 +97,9 @@ constexpr int kViscRefWarps = 4;  // reference-order viscosity sweep: one task p
 constexpr int kGridWarps = 4;
 constexpr int kScanThreads = 1024;
 constexpr int kScanTile = 4 * kScanThreads;  // scan positions per block
+// Grids of more tiles take a pass over the tiles' sums (k_tile_offsets, which
+// has the figures).
+constexpr int kScanFewTiles = 512;
 constexpr int kElemThreads = 256;  // elementwise kernels
 constexpr int kCollideThreads = 256;
 constexpr int kSpringWarps = 4;
@@ -127,6 +130,7 @@ __global__ void k_visc_boxes(Totals tt, Particles P, SimTables T);
 __global__ void k_viscosity_ref(Totals tt, Particles P, SimTables T);
 __global__ void k_predict(Totals tt, Particles P, SimTables T);
 __global__ void k_live_reduce(Totals tt, SimTables T);
+__global__ void k_tile_offsets(int *tiles, int ntiles);
 __global__ void k_live_apply(Totals tt, SimTables T);
 __global__ void k_scan_reduce(Totals tt, SimTables T);
 __global__ void k_scan_apply(Totals tt, SimTables T);
