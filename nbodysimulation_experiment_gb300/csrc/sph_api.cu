@@ -101,7 +101,6 @@ struct sph_sim {
 	cudaStream_t stream = nullptr;
 	int numSMs = 0;
 	int viscBlocks = 0, deltaBlocks = 0, densBlocks = 0, gridBlocks = 0;
-	int densSplit = 0;  // two warps per cell, see k_density
 	int viscLean = 0;   // viscosity shape: 0 = wide, 1 = lean (sph_kernels.cuh)
 	bool refOrder = false;  // sweeps and grid events in AddParticle order (sph_set_reference_order)
 	int viscRefBlocks = 0;
@@ -531,7 +530,11 @@ int enqueue_step(sph_sim *s, bool capturing) {
 	SimTables T = tables(s);
 	const int cellOrN = std::max(tt.n, tt.ncell);
 	bool anyCanonical = false;
-	for (const Scene &sc : s->scenes) anyCanonical = anyCanonical || sc.n0 > 0;
+	int added = tt.n;
+	for (const Scene &sc : s->scenes) {
+		anyCanonical = anyCanonical || sc.n0 > 0;
+		added -= (int)sc.n0;
+	}
 	// Under capture, stage events become event-record nodes of the graph.
 	auto mark = [&](int k) {
 		return capturing ? cudaEventRecordWithFlags(s->ev[k], st, cudaEventRecordExternal)
@@ -617,7 +620,7 @@ int enqueue_step(sph_sim *s, bool capturing) {
 	}
 	SPH_CUDA(mark(kEvSprings));
 
-	k_density<<<s->densBlocks, kDensWarps * kWarp, dens_smem_bytes(), st>>>(tt, B.view(), T, s->densSplit);
+	k_density<<<s->densBlocks, kDensWarps * kWarp, dens_smem_bytes(), st>>>(tt, B.view(), T, added, s->numSMs);
 	SPH_LAUNCHED(s);
 	SPH_CUDA(mark(kEvDensity));
 
@@ -910,8 +913,7 @@ int allocate(sph_sim *s) {
 		if (sweep_occupancy(false, kDeltaDense, &v2, &d2) != cudaSuccess || d2 < 1) return SPH_ERR_CUDA;
 		s->crowdedDeltaBlocks = d2 * s->numSMs;
 	}
-	s->densSplit = C <= 112 * s->numSMs ? 1 : 0;
-	s->densBlocks = std::max(1, std::min(blocks_for(C << s->densSplit, kDensWarps), 64 * s->numSMs));
+	s->densBlocks = std::max(1, std::min(blocks_for(2 * C, kDensWarps), 64 * s->numSMs));
 	s->springBlocks = std::max(1, std::min(blocks_for(C, kSpringWarps), 64 * s->numSMs));
 	s->gridBlocks = std::max(1, std::min(blocks_for(C, kGridWarps), 64 * s->numSMs));
 	s->viscRefBlocks = 8 * s->numSMs;
@@ -1120,7 +1122,7 @@ int density_error(sph_sim *s, float *out, uint32_t *maxNb = nullptr) {
 	Particles Q = s->buf[s->cur].view();
 	Q.dens = s->ldens;
 	Q.press = s->lbyId;
-	k_density<<<s->densBlocks, kDensWarps * kWarp, dens_smem_bytes(), s->stream>>>(tt, Q, T, s->densSplit);
+	k_density<<<s->densBlocks, kDensWarps * kWarp, dens_smem_bytes(), s->stream>>>(tt, Q, T, 0, s->numSMs);
 	SPH_LAUNCHED(s);
 	const int blocks = std::min(blocks_for(tt.n, kErrThreads), kErrBlocks);
 	k_density_error<<<blocks, kErrThreads, 0, s->stream>>>(tt.n, s->ldens, sc.params.rest_density, s->lerr);

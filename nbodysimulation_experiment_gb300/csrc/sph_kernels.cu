@@ -37,6 +37,7 @@
 #include "sph_internal.cuh"
 #include "sph_kernels.cuh"
 #include "sph_math.cuh"
+#include "sph_rules.h"
 
 namespace sphgb {
 
@@ -1716,13 +1717,12 @@ __global__ void k_app_boxes(Totals tt, SimTables T) {
 // Bound by instruction issue on large grids (1M block: 0.78 instructions per
 // cycle and scheduler, DRAM 0.3 %), so a cell, or the rest of one, of at most
 // 32 particles runs the loop with one list per lane instead of an empty second
-// one (128 scenes 0.81 -> 0.71 ms, 1M block 0.44 -> 0.43).  Small grids are
-// bound by one warp's time for its cell; with `split` two warps share a cell,
-// 32 particles each at a time: 4,096 dam break 52 -> 35 us, 65,536 particles
-// among obstacles 99 -> 66 us, where on the 1M block the staging done twice
-// costs more (0.43 -> 0.49 ms).  The host splits while two warps for each
-// occupied cell, about one cell in seven of the scenes here, are resident at
-// once at 32 warps per SM: 112 cells per SM.
+// one (128 scenes 0.81 -> 0.71 ms, 1M block 0.44 -> 0.43).  With few occupied
+// cells it is bound by one warp's time for its cell; there two warps share a
+// cell, 32 particles each at a time: 4,096 dam break 52 -> 35 us, 65,536
+// particles among obstacles 99 -> 66 us.  Where the warps of all cells are not
+// resident at once, the staging done twice costs more (1M block 0.43 -> 0.49 ms):
+// density_halves (sph_rules.h).
 
 constexpr int kDensChunk = 256;
 struct DensWarp {
@@ -1790,53 +1790,67 @@ __device__ __forceinline__ void dens_lists(DensWarp &S, const Particles &Q, cons
 	}
 }
 
+// The particles of cell c (cnt of them) from `first` on, 64 at a time: two
+// lists per lane or, as one of a cell's two warps (kHalf), every other 32.
+template <bool kHalf>
+__device__ __forceinline__ void dens_cell(DensWarp &S, const Particles &Q, const SimTables &T, int c, int cnt, int first,
+                                          int lane) {
+	const int sid = T.sceneOfCell[c];
+	const SceneDev &sc = T.scenes[sid];
+	const StepParams &s = sc.p;
+	const int base = sc.cellBase;
+	const int cx = (c - base) % s.gx, cy = (c - base) / s.gx;
+	int segStart[9], segOff[9];
+	int L = 0;
+#pragma unroll
+	for (int q = 0; q < 9; ++q) {
+		const int x = cx + q % 3 - 1, y = cy + q / 3 - 1;
+		int st = 0, nn = 0;
+		if (x >= 0 && x < s.gx && y >= 0 && y < s.gy) {
+			const int c2 = base + y * s.gx + x;
+			st = T.newStart[c2];
+			nn = T.newCount[c2];
+		}
+		segStart[q] = st;
+		segOff[q] = L;
+		L += nn;
+	}
+	if (lane == 0 && first == 0) {
+		atomicMin(&T.stats[4 * sid + 0], (uint32_t)L);
+		atomicMax(&T.stats[4 * sid + 1], (uint32_t)L);
+	}
+	if (L > kStageCap) {
+		if (lane == 0) atomicOr(T.error, kErrStageOverflow);
+		return;
+	}
+	const int st = T.newStart[c];
+	for (int g = first; g < cnt; g += 2 * kWarp) {
+		if (!kHalf && cnt - g > kWarp)
+			dens_lists<2>(S, Q, segOff, segStart, L, st, g + lane, cnt, s, lane);
+		else
+			dens_lists<1>(S, Q, segOff, segStart, L, st, g + lane, cnt, s, lane);
+	}
+	__syncwarp();
+}
+
 }  // namespace
 
-__global__ void __launch_bounds__(kDensWarps * kWarp, 4) k_density(Totals tt, Particles Q, SimTables T, int split) {
+__global__ void __launch_bounds__(kDensWarps * kWarp, 4) k_density(Totals tt, Particles Q, SimTables T, int added,
+                                                                   int sms) {
 	extern __shared__ __align__(16) unsigned char smem_raw[];
 	DensWarp &S = reinterpret_cast<DensWarp *>(smem_raw)[threadIdx.x / kWarp];
 	const int lane = threadIdx.x & (kWarp - 1);
-	const int warpsTotal = gridDim.x * kDensWarps;
-	for (int w = blockIdx.x * kDensWarps + threadIdx.x / kWarp; w < tt.ncell << split; w += warpsTotal) {
-		const int c = w >> split, first = (w & split) * kWarp;
-		const int cnt = T.newCount[c];
-		if (cnt <= first) continue;
-		const int sid = T.sceneOfCell[c];
-		const SceneDev &sc = T.scenes[sid];
-		const StepParams &s = sc.p;
-		const int base = sc.cellBase;
-		const int cx = (c - base) % s.gx, cy = (c - base) / s.gx;
-		int segStart[9], segOff[9];
-		int L = 0;
-#pragma unroll
-		for (int q = 0; q < 9; ++q) {
-			const int x = cx + q % 3 - 1, y = cy + q / 3 - 1;
-			int st = 0, nn = 0;
-			if (x >= 0 && x < s.gx && y >= 0 && y < s.gy) {
-				const int c2 = base + y * s.gx + x;
-				st = T.newStart[c2];
-				nn = T.newCount[c2];
-			}
-			segStart[q] = st;
-			segOff[q] = L;
-			L += nn;
+	const int warpsTotal = gridDim.x * kDensWarps, first = blockIdx.x * kDensWarps + threadIdx.x / kWarp;
+	if (density_halves(tt.ncell, *T.nLive, added, sms)) {
+		for (int w = first; w < 2 * tt.ncell; w += warpsTotal) {
+			const int cnt = T.newCount[w >> 1];
+			if (cnt > (w & 1) * kWarp) dens_cell<true>(S, Q, T, w >> 1, cnt, (w & 1) * kWarp, lane);
 		}
-		if (lane == 0 && first == 0) {
-			atomicMin(&T.stats[4 * sid + 0], (uint32_t)L);
-			atomicMax(&T.stats[4 * sid + 1], (uint32_t)L);
+	} else {
+		for (int c = first; c < tt.ncell; c += warpsTotal) {
+			const int cnt = T.newCount[c];
+			if (cnt > 0) dens_cell<false>(S, Q, T, c, cnt, 0, lane);
 		}
-		if (L > kStageCap) {
-			if (lane == 0) atomicOr(T.error, kErrStageOverflow);
-			continue;
-		}
-		const int st = T.newStart[c];
-		for (int g = first; g < cnt; g += 2 * kWarp) {
-			if (split == 0 && cnt - g > kWarp)
-				dens_lists<2>(S, Q, segOff, segStart, L, st, g + lane, cnt, s, lane);
-			else
-				dens_lists<1>(S, Q, segOff, segStart, L, st, g + lane, cnt, s, lane);
-		}
-		__syncwarp();
 	}
 }
 
