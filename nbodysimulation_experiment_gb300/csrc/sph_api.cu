@@ -87,11 +87,7 @@ struct Scene {
 	int cellBase = 0, pBase = 0, bodyBase = 0;  // offsets into the shared arrays
 	sph_spring_params springs{};
 	std::vector<float2> pendPos, pendForce;
-	// Runs of the particles added since the last update (appendix tasks): the
-	// number where the first begins, and where each ends.
-	size_t runFrom = 0;
-	std::vector<int> runEnd;
-	float2 runLast{};
+	AppendixRuns runs;  // of the particles added since the last update (appendix tasks)
 };
 
 }  // namespace
@@ -342,36 +338,11 @@ int ensure_stage(sph_sim *s, size_t count) {
 	return SPH_OK;
 }
 
-// Divide the `count` pending particles (numbers nDev onwards) into appendix
-// runs: kAppendixRun consecutive ones, or fewer where the next particle lies
-// far away, as at the end of a lattice row.  A run across that jump would have
-// a box as wide as the lattice: it would wait for, and hold up, every run of
-// two rows, and its region would outgrow the sweep's stage (30,011 particles
-// in rows of 174: delta sweep of the first update 26 against 7.8 ms).  At most one run per
-// sixteen particles in all, whatever their order.
+// The `count` pending particles (numbers nDev onwards) join the appendix runs.
 void extend_runs(Scene &sc, size_t count) {
-	if (sc.nDev == sc.n0) {
-		sc.runEnd.clear();
-		sc.runFrom = sc.n0;
-	}
-	if ((sc.runEnd.empty() ? sc.runFrom : (size_t)sc.runEnd.back()) != sc.nDev) return;  // unknown numbers: fixed runs
-	if (!sc.runEnd.empty()) sc.runEnd.pop_back();  // the last run goes on
-	size_t from = sc.runEnd.empty() ? sc.runFrom : (size_t)sc.runEnd.back();
-	const float far = 2.0f * sc.dom.cell_size;
-	float2 last = sc.nDev == sc.runFrom ? sc.pendPos[0] : sc.runLast;
-	for (size_t k = 0; k < count; ++k) {
-		const size_t i = sc.nDev + k;
-		const float2 p = sc.pendPos[k];
-		const bool jump = std::fabs(p.x - last.x) > far || std::fabs(p.y - last.y) > far;
-		if (i - from == (size_t)kAppendixRun ||
-		    (jump && i > from && (sc.runEnd.size() + 1) * (kAppendixRun / 2) <= i - sc.runFrom)) {
-			sc.runEnd.push_back((int)i);
-			from = i;
-		}
-		last = p;
-	}
-	sc.runLast = last;
-	sc.runEnd.push_back((int)(sc.nDev + count));
+	if (sc.nDev == sc.n0) sc.runs.restart(sc.n0);
+	if (sc.runs.end() != sc.nDev) return;  // unknown numbers: fixed runs
+	sc.runs.add(sc.pendPos.data(), count, sc.dom.cell_size);
 }
 
 // Pending AddParticle calls reach the device in order, before anything that
@@ -476,7 +447,7 @@ int check_device_errors(sph_sim *s) {
 	return SPH_OK;
 }
 
-// Appendix runs (particles added since the last update, extend_runs) of every
+// Appendix runs (particles added since the last update, AppendixRuns) of every
 // scene as delta-sweep tasks after the canonical ones,
 // interleaved across scenes; in reference order, runs of the whole scene in
 // AddParticle order are the only delta-sweep tasks.  A run waits for the earlier runs of its scene
@@ -493,8 +464,8 @@ int upload_appendix_tasks(sph_sim *s) {
 		const size_t first = s->refOrder ? 0 : sc.n0;
 		begin[k] = (int)first;
 		if (first == sc.nDev) continue;
-		if (!s->refOrder && sc.runFrom == first && !sc.runEnd.empty() && (size_t)sc.runEnd.back() == sc.nDev) {
-			ends[k] = sc.runEnd;
+		if (!s->refOrder && sc.runs.from == first && sc.runs.end() == sc.nDev) {
+			ends[k] = sc.runs.ends;
 		} else {
 			for (size_t e = first; e < sc.nDev;) ends[k].push_back((int)(e = std::min(e + kAppendixRun, sc.nDev)));
 		}
@@ -829,7 +800,7 @@ int allocate(sph_sim *s) {
 	    (rc = dalloc(&T.nLive, 1)) ||
 	    (rc = dalloc(&T.abort, 1)) || (rc = dalloc(&T.bodies, s->bodyCap)))
 		return rc;
-	// Appendix runs (extend_runs): at most one per kAppendixRun / 2 particles of a
+	// Appendix runs (AppendixRuns): at most one per kAppendixRun / 2 particles of a
 	// scene, and two more.
 	const size_t appCap = N / (kAppendixRun / 2) + 2 * S + 1;
 	s->doneDCap = C + appCap;

@@ -5,6 +5,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "sph_rules.h"
+
 namespace sphgb {
 
 constexpr int kWarp = 32;
@@ -32,9 +34,6 @@ constexpr int kCellCap = 512;
 constexpr int kRegionCells = 100;
 constexpr int kMaxBodies = 100;  // kSPHMaxBodyCount, sph.h:71
 constexpr int kMaxPoly = 8;      // kMaxScenarioPolygonCount, sph.h:161
-// Appendix particles (added since the last update) are swept serially in runs
-// of at most this many consecutive numbers.
-constexpr int kAppendixRun = 32;
 // Pending dependencies a delta-sweep task lists before one warp polls them.
 constexpr int kPendCap = 128;
 // Spring slots per particle (viscoelastic springs, not in the reference).

@@ -37,7 +37,6 @@
 #include "sph_internal.cuh"
 #include "sph_kernels.cuh"
 #include "sph_math.cuh"
-#include "sph_rules.h"
 
 namespace sphgb {
 
@@ -2475,6 +2474,12 @@ __device__ __forceinline__ int run_pipeline(DeltaSmemT<C> &S, int i, int n, int 
 // The longest run of particles from `k` on (at most 32) whose region, the
 // bounding box of their new cells grown by one, fits the stage; at least one
 // particle.  Warp 0; lane i looks at the box of the first i + 1 particles.
+// Particles added in no spatial order are groups of one, each with this on the
+// chain.  The first particle's region therefore is not counted (it goes in
+// whatever it holds), and the last warp, which has no cell of a single
+// particle's region to stage in the shapes with many warps, loads the group's
+// inputs: first update of 30,000 in random order 113 -> 98 ms, of 100,000 420 ->
+// 330.
 template <class C>
 __device__ __forceinline__ void next_group(DeltaSmemT<C> &S, int k, int p1, const int *ord, const SimTables &T,
                                            const StepParams &s, int cellBase, int tid) {
@@ -2496,7 +2501,7 @@ __device__ __forceinline__ void next_group(DeltaSmemT<C> &S, int k, int p1, cons
 	const int rx0 = max(x0 - 1, 0), ry0 = max(y0 - 1, 0), rx1 = min(x1 + 1, s.gx - 1), ry1 = min(y1 + 1, s.gy - 1);
 	bool fits = k + tid < p1 && (rx1 - rx0 + 1) * (ry1 - ry0 + 1) <= C::kRegion;
 	int entries = 0;
-	if (fits) {
+	if (fits && tid > 0) {
 		for (int y = ry0; y <= ry1; ++y)
 			for (int x = rx0; x <= rx1; ++x) entries += T.newCount[cellBase + y * s.gx + x];
 		fits = entries <= C::kStage;
@@ -2565,7 +2570,13 @@ __device__ __forceinline__ unsigned long long relax_group(DeltaSmemT<C> &S, int 
 			grow(box.x, box.y, box.z, box.w);
 			staged = stage_table<C>(S, R, T, s, cellBase, tid);
 			if (staged) {
-				inputs(g0, min(g1, g0 + C::kPrefetch));
+				const int k = g0 + lane;  // a group has at most 32
+				if (warp == C::kWarps - 1 && k < g1) {
+					const int q = ord ? ord[k] : k;
+					const int jk = T.newLabel[q], nc = T.newCell[q];
+					S.ppk[k - g0] = Q.press[jk];
+					particle_slots<C>(S, R, nc, jk, s, cellBase, T.error, S.pslot[k - g0], S.plen[k - g0]);
+				}
 				stage_positions<C>(S, R, Q, tid);
 			} else if (tid == 0) {
 				atomicOr(T.error, kErrStageOverflow);  // one 3x3 block alone

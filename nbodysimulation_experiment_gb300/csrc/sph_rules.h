@@ -2,7 +2,10 @@
 // the kernels and the tests.
 #pragma once
 
+#include <math.h>
 #include <stddef.h>
+
+#include <vector>
 
 #ifdef __CUDACC__
 #define SPH_RULE __host__ __device__ inline
@@ -27,5 +30,58 @@ SPH_RULE bool density_halves(int cells, int liveCells, int added, int sms) {
 	const int live = liveCells + added / 48;
 	return live <= 16 * sms ? cells <= 1728 * sms : live > 32 * sms && cells <= 48 * sms;
 }
+
+// Particles added since the last update are swept serially in runs of at most
+// this many consecutive numbers.
+constexpr int kAppendixRun = 32;
+
+// Divides a scene's added particles, in the order they come, into runs: fewer
+// than kAppendixRun of them where a particle lies far from the last one and the
+// next kStretch near one another, as at the end of a lattice row.  A run across
+// that jump would have a box as wide as the lattice: it would wait for, and hold
+// up, every run of two rows, and its region would outgrow the sweep's stage
+// (30,011 particles in rows of 174: delta sweep of the first update 26 against
+// 7 ms).  Where the next ones are far again, as in a random order, another end
+// only adds a run (30,000 in random order: 118 against 113 ms).  At most one run
+// per sixteen particles in all, whatever their order.
+class AppendixRuns {
+public:
+	size_t from = 0;        // the first run's first number
+	std::vector<int> ends;  // where each run ends
+	size_t end() const { return ends.empty() ? from : (size_t)ends.back(); }
+	void restart(size_t first) {
+		from = first;
+		ends.clear();
+		jump = first;
+	}
+	// `count` more particles at pos, numbers end() onwards.
+	template <class V>
+	void add(const V *pos, size_t count, float cellSize) {
+		const size_t first = end();
+		if (count == 0) return;
+		if (!ends.empty()) ends.pop_back();  // the last run goes on
+		size_t start = end();
+		const float far = 2.0f * cellSize;
+		for (size_t k = 0; k < count; ++k) {
+			const size_t i = first + k;
+			const bool near = i != from && fabsf(pos[k].x - lastX) <= far && fabsf(pos[k].y - lastY) <= far;
+			if (!near) jump = i;
+			lastX = pos[k].x;
+			lastY = pos[k].y;
+			// A full run ends at a jump just before, if there is one.
+			const bool full = i - start == (size_t)kAppendixRun, recent = jump > start && i - jump <= kStretch;
+			if (full || (recent && i - jump == kStretch && (ends.size() + 1) * (kAppendixRun / 2) <= jump - from)) {
+				start = recent ? jump : i;
+				ends.push_back((int)start);
+			}
+		}
+		ends.push_back((int)(first + count));
+	}
+
+private:
+	static constexpr size_t kStretch = 3;
+	size_t jump = 0;  // the last particle far from the one before (none yet: from)
+	float lastX = 0.0f, lastY = 0.0f;
+};
 
 }  // namespace sphgb

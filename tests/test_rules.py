@@ -3,6 +3,7 @@ import ctypes
 import os
 import subprocess
 
+import numpy as np
 import pytest
 
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
@@ -10,6 +11,15 @@ SHIM = r"""
 #include "sph_rules.h"
 using namespace sphgb;
 extern "C" {
+struct P { float x, y; };
+// The runs' ends of the particles at xy, added in batches of the given counts.
+int runs(const P *xy, const int *batch, int batches, int first, float cell, int *ends) {
+	AppendixRuns r;
+	r.restart(first);
+	for (int b = 0; b < batches; xy += batch[b++]) r.add(xy, batch[b], cell);
+	for (size_t k = 0; k < r.ends.size(); ++k) ends[k] = r.ends[k];
+	return (int)r.ends.size();
+}
 int halves(int cells, int live, int added, int sms) { return density_halves(cells, live, added, sms); }
 }
 """
@@ -40,3 +50,83 @@ def rules(tmp_path_factory):
 ])
 def test_density_halves(rules, cells, live, added, want):
     assert rules.halves(cells, live, added, 152) == want
+
+
+RUN = 32
+CELL = 0.3
+
+
+def _runs(rules, pos, batches=None, first=0):
+    pos = np.ascontiguousarray(pos, np.float32)
+    batches = np.array([len(pos)] if batches is None else batches, np.int32)
+    assert batches.sum() == len(pos)
+    ends = np.zeros(len(pos) + 1, np.int32)
+    rules.runs.argtypes = [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_int, ctypes.c_int, ctypes.c_float, ctypes.c_void_p]
+    k = rules.runs(pos.ctypes.data, batches.ctypes.data, len(batches), first, CELL, ends.ctypes.data)
+    ends = ends[:k] - first
+    starts = np.concatenate([[0], ends[:-1]])
+    assert ends[-1] == len(pos) and (ends > starts).all() and (ends - starts <= RUN).all()  # a partition
+    assert k <= len(pos) // (RUN // 2) + 2  # what the run arrays hold
+    return ends
+
+
+def _rows(width, rows):
+    y, x = np.divmod(np.arange(width * rows), width)
+    return np.stack([x, y], 1) * 0.05
+
+
+def test_runs_end_with_lattice_rows(rules):
+    ends = _runs(rules, _rows(174, 40))
+    assert set(range(174, 174 * 40, 174)) <= set(ends.tolist())
+    assert len(ends) == 6 * 40
+
+
+@pytest.mark.parametrize("width", [29, 30, 31, 32, 33, 61, 63, 65])
+def test_runs_end_with_rows_about_as_long_as_a_run(rules, width):
+    """Also where the run would be full just past the row's end."""
+    ends = _runs(rules, _rows(width, 30))
+    assert set(range(width, width * 29, width)) <= set(ends.tolist())
+
+
+@pytest.mark.parametrize("n", [1, 31, 32, 33, 3000])
+def test_runs_in_no_spatial_order_are_full(rules, n):
+    """A jump at every particle ends no run early."""
+    y, x = np.divmod(np.random.default_rng(n).permutation(n), 60)
+    assert len(_runs(rules, np.stack([x, y], 1) * (2.1 * CELL))) == -(-n // RUN)
+
+
+def test_runs_of_a_shuffled_block_are_almost_full(rules):
+    """Few are near the one before by chance."""
+    pos = np.random.default_rng(7).permutation(_rows(174, 174))
+    assert len(_runs(rules, pos)) <= 1.05 * len(pos) / RUN
+
+
+def test_runs_of_alternating_sources_are_full(rules):
+    a = np.arange(500) * 0.02
+    pos = np.stack([np.stack([a, a], 1), np.stack([a + 30.0, a], 1)], 1).reshape(-1, 2)
+    assert len(_runs(rules, pos)) == -(-1000 // RUN)
+
+
+@pytest.mark.parametrize("pos", [_rows(174, 20), _rows(33, 60), _rows(9, 100),
+                                 np.random.default_rng(1).uniform(-40.0, 40.0, (1000, 2)),
+                                 np.random.default_rng(2).uniform(-1.0, 1.0, (1000, 2))])
+def test_runs_do_not_depend_on_the_batches(rules, pos):
+    whole = _runs(rules, pos)
+    n = len(pos)
+    for batches in ([1] * n, [n // 3, 0, n - n // 3], [174] * (n // 174) + [n % 174]):
+        assert np.array_equal(_runs(rules, pos, batches), whole)
+    assert np.array_equal(_runs(rules, pos, first=12345), whole)
+
+
+@pytest.mark.parametrize("width", [2, 3, 4, 5, 7, 13, 15, 16, 17, 31, 33, 47])
+def test_runs_of_short_stretches_stay_within_their_number(rules, width):
+    """Stretches of `width` near particles, each far from the one before."""
+    k = np.arange(4000)
+    _runs(rules, np.stack([k // width * 10.0 % 70.0, k % width * 0.05 + k // width * 0.01], 1))
+
+
+def test_runs_of_odd_positions(rules):
+    pos = np.random.default_rng(3).uniform(-1.0, 1.0, (200, 2))
+    pos[50:60] = np.nan
+    pos[100:110] = np.inf
+    _runs(rules, pos)
