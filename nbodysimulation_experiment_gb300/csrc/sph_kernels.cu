@@ -640,14 +640,20 @@ __device__ __forceinline__ void st_release_cta(uint32_t *p, uint32_t v) {
 
 // Bounded wait of a producer warp until the chain has finished `count`
 // segments of slot s (a segment takes some 5 us).  False when it gave up, with
-// kErrTimeout and the abort flag raised.  Polled every 500 ns: more often, the
-// polling slowed the chains (2.67 against 2.88 ms on the 1M block).
-constexpr uint32_t kTakenPolls = 1u << 22;
+// kErrTimeout and the abort flag raised, or saw the abort flag.  Polled every
+// 500 ns: more often, the polling slowed the chains (2.67 against 2.88 ms on the
+// 1M block), as did reading the global timer.  So waitLimitNs is counted in
+// polls, as 512 ns each, and looked at with the abort flag at every eighth
+// (2.18 -> 2.19 ms; at every poll 2.23).
 template <class C>
 __device__ __forceinline__ bool slot_taken(ViscMultiSmemT<C> &S, int s, uint32_t count, const SimTables &T) {
-	for (uint32_t it = 0; it < kTakenPolls; ++it) {
+	for (uint32_t it = 0; it < kWaitLimitIter; ++it) {
 		const bool ok = (int)(ld_acquire_cta(&S.taken[s]) - count) >= 0;
 		if (__all_sync(kFull, ok)) return true;
+		if ((it & 7u) == 7u) {
+			if (__any_sync(kFull, ld_acquire(T.abort) != 0u)) return false;
+			if ((unsigned long long)it << 9 > T.waitLimitNs) break;
+		}
 		__nanosleep(500);
 	}
 	if ((threadIdx.x & (kWarp - 1)) == 0) {
@@ -723,7 +729,11 @@ __device__ __forceinline__ bool slot_entries(ViscMultiSmemT<C> &S, int s, ViscSe
 // depends on the finished pairs (the velocity to store, the next particle's
 // own and its first partners') follows at the end, in the turns where a lane
 // changes.
+// The loop ends once every producer has, and each of their waits is bounded;
+// after kChainTurns turns (some 80 s) it ends anyway, and a producer that still
+// waits for a segment reports the timeout.
 constexpr int kChainGroup = 4;
+constexpr uint32_t kChainTurns = 1u << 28;
 template <class C>
 __device__ __forceinline__ void slot_chains(ViscMultiSmemT<C> &S, int first, int lane) {
 	constexpr int kLanes = C::kSlots / C::kChains, U = kChainGroup;
@@ -756,7 +766,7 @@ __device__ __forceinline__ void slot_chains(ViscMultiSmemT<C> &S, int first, int
 	geometry(ga, at, end);
 	geometry(gb, at, end);
 	partners(va, ga);
-	for (uint32_t it = 0;; ++it) {
+	for (uint32_t it = 0; it < kChainTurns; ++it) {
 		if ((it & 15u) == 0u && !__any_sync(kFull, active)) {
 			if (*(volatile int *)&S.exited == C::kSlots) break;
 			__nanosleep(64);
