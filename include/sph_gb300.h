@@ -334,10 +334,11 @@ int sph_get_sweep_shape(sph_sim *sim, int *shape);
 int sph_set_sweep_shape(sph_sim *sim, const int *shape);
 
 /* Dense states.  With adaptive shapes on (the default), an update whose
- * previous updates saw neighbour lists longer than 555 runs the wide
- * viscosity shape, and one whose fullest cell held more than 120 particles
- * runs the 8-warp delta shape (4,096 staged entries), or the 16-warp shape
- * (12,288) past 145, instead of the tuned shapes (results are identical in
+ * previous updates saw neighbour lists longer than 520 runs the wide
+ * viscosity shape, and one whose fullest cell held more than 90 (lean), 108
+ * (tri) or 132 particles (quad) runs the 8-warp delta shape (4,096 staged
+ * entries), or any the 16-warp shape (12,288) past 150, instead of the tuned
+ * shapes (results are identical in
  * every shape; only the launch differs).  Single-scene simulations only: a
  * batch keeps its tuned shapes.  The statistics come from the
  * end of earlier updates, read without waiting.  sph_last_sweep_shape

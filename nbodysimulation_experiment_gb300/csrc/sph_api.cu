@@ -617,19 +617,25 @@ int enqueue_step(sph_sim *s, bool capturing) {
 }
 
 // Where dense states change shapes: measured crossovers on the collapsing 1M
-// column, whose other scenes' lie no lower.  Viscosity, longest neighbour list
-// of 542: lean 4.12 against wide 4.31 ms, of 577: 4.66 against 4.33.
-constexpr uint32_t kDenseNeighbors = 555;
-// Delta sweep, fullest cell of 117 particles: quad 3.97 against mid 4.10 ms, of
-// 138: 5.12 against 4.73 (tri from about 100).
-constexpr uint32_t kDenseCell = 120;
-// Fullest cell of 139: mid 6.21 against dense 6.29, of 162: 7.52 against 7.11.
-constexpr uint32_t kCrowdedCell = 145;
+// column, plain / with springs.  On the 65,536- and 262,144-particle scenes
+// among obstacles, whose colour levels hold fewer tasks, the wide viscosity and
+// the larger delta shapes are faster from the first updates on.
+// Viscosity, longest neighbour list: of 510 lean 3.82 against wide 4.00 ms, of 540
+// 4.46 against 4.00 / of 496 3.59 against 4.01, of 537 4.15 against 4.00.
+constexpr uint32_t kDenseNeighbors = 520;
+// Delta sweep, fullest cell, against mid (kDenseCell of each shape): lean, of 89
+// particles 3.46 and 3.60 ms, of 94 3.59 and 3.60 / of 82 3.23 and 3.62, of 86 3.73
+// and 3.64; tri, of 102 3.60 and 3.70, of 115 3.97 and 3.76 / of 105 3.40 and
+// 3.70, of 121 4.65 and 4.08; quad, of 129 4.25 and 4.33, of 138 5.64 and 5.23 / of
+// 121 3.72 and 4.08, of 154 4.83 and 4.66.
+// Mid against dense: of 138 5.23 and 5.74, of 148 7.01 and 6.84 / of 154 4.66 and
+// 5.51, of 163 8.07 and 7.74.
+constexpr uint32_t kCrowdedCell = 150;
 
 // The sweep shapes of the next update: the tuned ones, or in dense states
-// (see sph_sim::adaptive) the wide viscosity shape and, where the tuned delta
-// shape's stage is smaller, the 8-warp shape (4,096 entries) or, more crowded
-// still, the 16-warp shape (12,288 entries).  The statistics are those of the
+// (see sph_sim::adaptive) the wide viscosity shape and, for the smaller delta
+// shapes, the 8-warp shape (4,096 entries) or, more crowded still, the 16-warp
+// shape (12,288 entries).  The statistics are those of the
 // update before last at the latest: the host waits for its copy, so it never
 // runs more than two updates ahead.  Changing shapes drops the update graphs.
 void choose_shapes(sph_sim *s) {
@@ -648,17 +654,17 @@ void choose_shapes(sph_sim *s) {
 		}
 		// Hysteresis: back to the tuned shape only well below the threshold.
 		s->denseVisc = s->denseVisc ? maxNb * 5 > kDenseNeighbors * 4 : maxNb > kDenseNeighbors;
-		const uint32_t cap = (uint32_t)delta_stage_capacity(ds);
-		s->denseDelta = maxCell * (s->denseDelta ? 5u : 4u) > kDenseCell * 4u;
+		const uint32_t denseCell = delta_dense_cell(ds);
+		s->denseDelta = denseCell > 0 && maxCell * (s->denseDelta ? 5u : 4u) > denseCell * 4u;
 		s->crowdedDelta = maxCell * (s->crowdedDelta ? 5u : 4u) > kCrowdedCell * 4u;
 		if (vl && s->denseVisc) {
 			vl = 0;
 			vb = s->denseViscBlocks;
 		}
-		if (cap < (uint32_t)kDeltaDenseStageCap && s->crowdedDelta) {
+		if (ds != kDeltaDense && s->crowdedDelta) {
 			ds = kDeltaDense;
 			db = s->crowdedDeltaBlocks;
-		} else if (cap < (uint32_t)kDeltaStageCap && s->denseDelta) {
+		} else if (s->denseDelta) {
 			ds = kDeltaMid;
 			db = s->denseDeltaBlocks;
 		}

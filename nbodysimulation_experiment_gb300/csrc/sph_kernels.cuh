@@ -35,7 +35,8 @@ struct ViscLean {
 // compacted first (fewest square roots and divisions, for the shapes with two
 // or three producer warps: evaluated directly, tri took 1,853 ns per particle
 // of one task alone against 1,445, quad 1,234 against 1,148).  kApart: the
-// summer has its scheduler to itself (pipeline_role).
+// summer has its scheduler to itself (pipeline_role).  kDenseCell: particles in
+// the fullest cell from which the mid shape is faster (choose_shapes).
 struct DeltaWide {
 	static constexpr int kName = 12;
 	static constexpr int kWarps = 16, kProducers = 12, kStage = kDeltaStageCap, kChainW = 96, kPrefetch = 128, kMinBlocks = 1;
@@ -43,7 +44,7 @@ struct DeltaWide {
 	static constexpr bool kPipelined = true, kDirect = true, kApart = true;
 };
 struct DeltaLean {
-	static constexpr int kName = 2;
+	static constexpr int kName = 2, kDenseCell = 90;
 	static constexpr int kWarps = 2, kProducers = 1, kStage = 1760, kChainW = 192, kPrefetch = 64, kMinBlocks = 8;
 	static constexpr int kRegion = kRegionCells;
 	static constexpr bool kPipelined = false, kDirect = false, kApart = false;
@@ -60,13 +61,13 @@ struct DeltaMid {
 // many tasks run at once rather than by one task's latency: two (tri) or
 // three (quad) producer warps and the summer warp, several blocks per SM.
 struct DeltaTri {
-	static constexpr int kName = 3;
+	static constexpr int kName = 3, kDenseCell = 108;
 	static constexpr int kWarps = 3, kProducers = 2, kStage = 2000, kChainW = 256, kPrefetch = 64, kMinBlocks = 5;
 	static constexpr int kRegion = kRegionCells;
 	static constexpr bool kPipelined = true, kDirect = false, kApart = false;
 };
 struct DeltaQuad {
-	static constexpr int kName = 4;
+	static constexpr int kName = 4, kDenseCell = 132;
 	static constexpr int kWarps = 4, kProducers = 3, kStage = 3072, kChainW = 192, kPrefetch = 128, kMinBlocks = 4;
 	static constexpr int kRegion = kRegionCells;
 	static constexpr bool kPipelined = true, kDirect = false, kApart = true;
@@ -109,15 +110,13 @@ struct DensWarp;
 // The two ordered sweeps in a chosen shape (lean or wide), and their set-up.
 cudaError_t sweep_attributes();
 cudaError_t sweep_occupancy(bool viscLean, int deltaShape, int *occV, int *occD);
-// Staged entries of a delta-sweep task region in the given shape; larger
-// regions are swept unstaged (from global memory).
-inline int delta_stage_capacity(int shape) {
-	return shape == kDeltaLean    ? DeltaLean::kStage
-	       : shape == kDeltaMid   ? DeltaMid::kStage
-	       : shape == kDeltaTri   ? DeltaTri::kStage
-	       : shape == kDeltaQuad  ? DeltaQuad::kStage
-	       : shape == kDeltaDense ? DeltaDense::kStage
-	                              : DeltaWide::kStage;
+// The fullest cell's particles past which dense states leave a delta shape for
+// the mid one; 0: they do not (wide, mid, dense).
+inline uint32_t delta_dense_cell(int shape) {
+	return shape == kDeltaLean   ? DeltaLean::kDenseCell
+	       : shape == kDeltaTri  ? DeltaTri::kDenseCell
+	       : shape == kDeltaQuad ? DeltaQuad::kDenseCell
+	                             : 0;
 }
 void launch_viscosity(bool lean, int blocks, cudaStream_t st, Totals tt, Particles P, SimTables T);
 void launch_delta(int shape, int blocks, cudaStream_t st, Totals tt, Particles Q, SimTables T);
