@@ -2007,54 +2007,50 @@ int sph_autotune(sph_sim *s, float dt, int *shape) {
 	s->adaptive = false;  // time the shapes as given
 	rc = copy_state(s, true);
 	if (rc) return rc;
-	// Median of three timed updates per shape (after one warm-up update); the
-	// current shape is kept unless another is faster by more than 2%.
-	auto measure = [&](int vLean, int vBlocks, int dShape, int dBlocks, float *tv, float *td) -> int {
-		s->viscLean = vLean;
-		s->viscBlocks = vBlocks;
-		s->deltaShape = dShape;
-		s->deltaBlocks = dBlocks;
-		float v[3], d[3];
+	// Three timed updates per trial, after one warm-up update.
+	auto measure = [&](const SweepTrial &t, std::vector<float> &tv, std::vector<float> &td) -> int {
+		s->viscLean = t.viscLean;
+		s->viscBlocks = t.viscBlocks;
+		s->deltaShape = t.deltaShape;
+		s->deltaBlocks = t.deltaBlocks;
 		for (int rep = 0; rep < 4; ++rep) {
 			int r = copy_state(s, false);
 			if (!r) r = run_step(s, dt);
 			if (!r) r = check_device_errors(s);
 			if (r) return r;
 			if (rep == 0) continue;
-			SPH_CUDA(cudaEventElapsedTime(&v[rep - 1], s->ev[kEvIntegrate], s->ev[kEvVisc]));
-			SPH_CUDA(cudaEventElapsedTime(&d[rep - 1], s->ev[kEvDensity], s->ev[kEvDelta]));
+			float v = 0.f, d = 0.f;
+			SPH_CUDA(cudaEventElapsedTime(&v, s->ev[kEvIntegrate], s->ev[kEvVisc]));
+			SPH_CUDA(cudaEventElapsedTime(&d, s->ev[kEvDensity], s->ev[kEvDelta]));
+			tv.push_back(v);
+			td.push_back(d);
 		}
-		std::sort(v, v + 3);
-		std::sort(d, d + 3);
-		*tv = v[1];
-		*td = d[1];
 		return SPH_OK;
 	};
 	int pick[4] = {s->viscLean, s->viscBlocks, s->deltaShape, s->deltaBlocks};
-	float bestV = 0.f, bestD = 0.f;
-	rc = measure(pick[0], pick[1], pick[2], pick[3], &bestV, &bestD);
-	// Candidates: every delta shape, each timed with the viscosity shape of
-	// the same kind (lean with lean, wide with both pipelined delta shapes),
-	// at every resident block count per SM.
-	for (int dShape = 0; dShape < kDeltaShapes && !rc; ++dShape) {
-		const int lean = dShape == kDeltaLean ? 1 : 0;
-		int occV = 0, occD = 0;
-		rc = cuda_status(sweep_occupancy(lean != 0, dShape, &occV, &occD));
-		const int maxPer = std::max(occV, occD);
-		for (int per = 1; per <= maxPer && !rc; ++per) {
-			const int vb = std::min(per, occV) * s->numSMs, db = std::min(per, occD) * s->numSMs;
-			float tv = 0.f, td = 0.f;
-			rc = measure(lean, vb, dShape, db, &tv, &td);
-			if (rc) break;
-			if (tv < 0.98f * bestV) {
-				bestV = tv;
-				pick[0] = lean;
-				pick[1] = vb;
-			}
-			if (td < 0.98f * bestD) {
-				bestD = td;
-				pick[2] = dShape;
-				pick[3] = db;
+	int occV[2] = {0, 0}, occD[kDeltaShapes] = {};
+	for (int d = 0; d < kDeltaShapes && !rc; ++d) {
+		const int lean = d == kDeltaLean ? 1 : 0;
+		rc = cuda_status(sweep_occupancy(lean != 0, d, &occV[lean], &occD[d]));
+	}
+	if (!rc) {
+		const std::vector<SweepTrial> trials =
+		    sweep_trials({pick[0], pick[1], pick[2], pick[3]}, occV, occD, kDeltaShapes, kDeltaLean, s->numSMs);
+		std::vector<std::vector<float>> tv(trials.size()), td(trials.size());
+		for (size_t k = 0; k < trials.size() && !rc; ++k) rc = measure(trials[k], tv[trials[k].visc], td[trials[k].delta]);
+		if (!rc) {
+			while (tv.back().empty()) tv.pop_back();
+			while (td.back().empty()) td.pop_back();
+			const int v = pick_launch(std::move(tv)), d = pick_launch(std::move(td));
+			for (const SweepTrial &t : trials) {
+				if (t.visc == v) {
+					pick[0] = t.viscLean;
+					pick[1] = t.viscBlocks;
+				}
+				if (t.delta == d) {
+					pick[2] = t.deltaShape;
+					pick[3] = t.deltaBlocks;
+				}
 			}
 		}
 	}

@@ -5,6 +5,8 @@
 #include <math.h>
 #include <stddef.h>
 
+#include <algorithm>
+#include <utility>
 #include <vector>
 
 #ifdef __CUDACC__
@@ -83,5 +85,58 @@ private:
 	size_t jump = 0;  // the last particle far from the one before (none yet: from)
 	float lastX = 0.0f, lastY = 0.0f;
 };
+
+// One trial of the sweep autotuner: an update in these shapes.  visc and delta
+// number the sweeps' distinct launches in order of appearance.
+struct SweepTrial {
+	int viscLean, viscBlocks, deltaShape, deltaBlocks;
+	int visc = 0, delta = 0;
+};
+
+// The trials: the current shapes, then every delta shape at every resident block
+// count per SM up to the larger occupancy, each with the viscosity shape of the
+// same kind (lean with lean, wide with the pipelined ones).  occV: blocks per SM
+// of the wide and lean viscosity; occD: of the delta shapes.
+inline std::vector<SweepTrial> sweep_trials(SweepTrial current, const int (&occV)[2], const int *occD, int deltaShapes,
+                                            int leanShape, int sms) {
+	std::vector<SweepTrial> trials;
+	int viscs = 0, deltas = 0;
+	auto add = [&](SweepTrial t) {
+		t.visc = t.delta = -1;
+		for (const SweepTrial &e : trials) {
+			if (e.viscLean == t.viscLean && e.viscBlocks == t.viscBlocks) t.visc = e.visc;
+			if (e.deltaShape == t.deltaShape && e.deltaBlocks == t.deltaBlocks) t.delta = e.delta;
+		}
+		if (t.visc < 0) t.visc = viscs++;
+		if (t.delta < 0) t.delta = deltas++;
+		trials.push_back(t);
+	};
+	add(current);
+	for (int d = 0; d < deltaShapes; ++d) {
+		const int lean = d == leanShape ? 1 : 0;
+		for (int per = 1; per <= std::max(occV[lean], occD[d]); ++per)
+			add({lean, std::min(per, occV[lean]) * sms, d, std::min(per, occD[d]) * sms});
+	}
+	return trials;
+}
+
+// The launch to keep from each launch's times: the first (the current one) unless
+// another's median is faster by more than 2%.  All times of a launch count once,
+// however many trials ran it: the lean viscosity, one block per SM, runs in
+// eight of them, and the fastest of eight draws would be held against the only
+// one of others.
+inline int pick_launch(std::vector<std::vector<float>> times) {
+	int best = 0;
+	float bestTime = 0.0f;
+	for (size_t k = 0; k < times.size(); ++k) {
+		std::vector<float> &t = times[k];
+		std::sort(t.begin(), t.end());
+		const float median = 0.5f * (t[(t.size() - 1) / 2] + t[t.size() / 2]);
+		if (k > 0 && !(median < 0.98f * bestTime)) continue;
+		best = (int)k;
+		bestTime = median;
+	}
+	return best;
+}
 
 }  // namespace sphgb

@@ -20,6 +20,22 @@ int runs(const P *xy, const int *batch, int batches, int first, float cell, int 
 	for (size_t k = 0; k < r.ends.size(); ++k) ends[k] = r.ends[k];
 	return (int)r.ends.size();
 }
+// The trials as rows of six numbers.
+int trials(const int *now, const int *occV, const int *occD, int shapes, int lean, int sms, int *out) {
+	const int v[2] = {occV[0], occV[1]};
+	int n = 0;
+	for (const SweepTrial &t : sweep_trials({now[0], now[1], now[2], now[3]}, v, occD, shapes, lean, sms)) {
+		const int row[6] = {t.viscLean, t.viscBlocks, t.deltaShape, t.deltaBlocks, t.visc, t.delta};
+		for (int k = 0; k < 6; ++k) out[6 * n + k] = row[k];
+		++n;
+	}
+	return n;
+}
+int pick(const float *times, const int *counts, int n) {
+	std::vector<std::vector<float>> t(n);
+	for (int k = 0; k < n; times += counts[k++]) t[k].assign(times, times + counts[k]);
+	return pick_launch(t);
+}
 int halves(int cells, int live, int added, int sms) { return density_halves(cells, live, added, sms); }
 }
 """
@@ -130,3 +146,39 @@ def test_runs_of_odd_positions(rules):
     pos[50:60] = np.nan
     pos[100:110] = np.inf
     _runs(rules, pos)
+
+
+@pytest.mark.parametrize("now", [(0, 608, 0, 152), (1, 152, 3, 760), (0, 7, 2, 9)])
+@pytest.mark.parametrize("occ_v, occ_d", [((4, 1), (1, 8, 2, 5, 4, 1)), ((4, 3), (1, 6, 2, 1, 1, 9))])
+def test_trials_number_the_distinct_launches(rules, now, occ_v, occ_d):
+    i32 = ctypes.c_int
+    out = (i32 * 6000)()
+    n = rules.trials((i32 * 4)(*now), (i32 * 2)(*occ_v), (i32 * 6)(*occ_d), 6, 1, 152, out)
+    rows = np.array(out[:6 * n]).reshape(n, 6)
+    assert tuple(rows[0]) == now + (0, 0)
+    # As many trials as the larger occupancy of each pair of shapes.
+    assert n == 1 + sum(max(occ_v[d == 1], occ_d[d]) for d in range(6))
+    want_v = {now[:2]} | {(0, 152 * k) for k in range(1, occ_v[0] + 1)} | {(1, 152 * k) for k in range(1, occ_v[1] + 1)}
+    want_d = {now[2:]} | {(d, 152 * k) for d in range(6) for k in range(1, occ_d[d] + 1)}
+    for launches, ids, want in ((rows[:, 0:2], rows[:, 4], want_v), (rows[:, 2:4], rows[:, 5], want_d)):
+        number = {}
+        for p, k in zip(map(tuple, launches), ids):
+            assert number.setdefault(p, len(number)) == k
+        assert set(number) == want
+
+
+def _pick(rules, times):
+    flat = np.array([x for t in times for x in t], np.float32)
+    counts = np.array([len(t) for t in times], np.int32)
+    rules.pick.argtypes = [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_int]
+    return rules.pick(flat.ctypes.data, counts.ctypes.data, len(times))
+
+
+def test_pick_counts_each_launch_once(rules):
+    assert _pick(rules, [[1.0] * 3, [0.97] * 3]) == 1
+    assert _pick(rules, [[1.0] * 3, [0.985] * 3]) == 0               # within 2%
+    assert _pick(rules, [[1.0] * 3, [0.9] * 3, [0.8] * 3, [0.79] * 3]) == 2
+    # One fast draw of many does not make a launch faster, one slow draw not slower.
+    many = [1.0] * 23 + [0.5]
+    assert _pick(rules, [[0.99] * 3, many]) == 0
+    assert _pick(rules, [[1.0] * 3, [0.9, 0.9, 5.0]]) == 1
