@@ -1850,7 +1850,7 @@ __global__ void __launch_bounds__(kDensWarps * kWarp, 4) k_density(Totals tt, Pa
 	DensWarp &S = reinterpret_cast<DensWarp *>(smem_raw)[threadIdx.x / kWarp];
 	const int lane = threadIdx.x & (kWarp - 1);
 	const int warpsTotal = gridDim.x * kDensWarps, first = blockIdx.x * kDensWarps + threadIdx.x / kWarp;
-	if (density_halves(tt.ncell, *T.nLive, added, sms)) {
+	if (density_halves(tt.ncell, *T.nLive, tt.n, added, sms)) {
 		for (int w = first; w < 2 * tt.ncell; w += warpsTotal) {
 			const int cnt = T.newCount[w >> 1];
 			if (cnt > (w & 1) * kWarp) dens_cell<true>(S, Q, T, w >> 1, cnt, (w & 1) * kWarp, lane);

@@ -36,7 +36,7 @@ int pick(const float *times, const int *counts, int n) {
 	for (int k = 0; k < n; times += counts[k++]) t[k].assign(times, times + counts[k]);
 	return pick_launch(t);
 }
-int halves(int cells, int live, int added, int sms) { return density_halves(cells, live, added, sms); }
+int halves(int cells, int live, int n, int added, int sms) { return density_halves(cells, live, n, added, sms); }
 }
 """
 
@@ -51,21 +51,22 @@ def rules(tmp_path_factory):
     return ctypes.CDLL(so)
 
 
-@pytest.mark.parametrize("cells, live, added, want", [
-    (1590, 114, 0, 1),        # the 4,096-particle dam break in its box
-    (262144, 120, 0, 1),      # a small scene in a large box
-    (2400, 2400, 0, 1),
-    (16500, 16500, 0, 0),     # a full box
-    (3000, 3000, 0, 0),
-    (4864, 4800, 0, 0),
-    (6000, 6000, 0, 1),       # a last wave nearly empty with one warp a cell
-    (65280, 6000, 0, 0),
-    (1048576, 120, 0, 0),     # mostly empty cells to pass over
-    (1590, 0, 4096, 1),       # the same scenes' first updates
-    (16500, 0, 594000, 0),
+@pytest.mark.parametrize("cells, live, n, added, want", [
+    (1590, 114, 4096, 0, 1),          # the 4,096-particle dam break in its box
+    (262144, 120, 4320, 0, 1),        # a small scene in a large box
+    (2400, 2400, 86400, 0, 1),
+    (16320, 3000, 65536, 0, 1),       # a spread-out block: few cells hold more than 32
+    (16500, 16500, 594000, 0, 0),     # a full box
+    (3000, 3000, 108000, 0, 0),
+    (4864, 4800, 172800, 0, 0),
+    (6000, 6000, 216000, 0, 1),       # a last wave nearly empty with one warp a cell
+    (65280, 6000, 216000, 0, 0),
+    (1048576, 120, 4320, 0, 0),       # mostly empty cells to pass over
+    (1590, 0, 4096, 4096, 1),         # the same scenes' first updates
+    (16500, 0, 594000, 594000, 0),
 ])
-def test_density_halves(rules, cells, live, added, want):
-    assert rules.halves(cells, live, added, 152) == want
+def test_density_halves(rules, cells, live, n, added, want):
+    assert rules.halves(cells, live, n, added, 152) == want
 
 
 RUN = 32
