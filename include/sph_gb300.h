@@ -201,7 +201,10 @@ int sph_load_state(sph_sim *sim, const sph_state_view *in);
 /* The simulation's CUDA stream (cudaStream_t) and device arrays, for callers
  * that time on the stream or consume results on the device.  Device arrays
  * are float2 in the internal numbering and are valid until the next call
- * that changes the simulation. */
+ * that changes the simulation.  sph_update only enqueues its work on that
+ * stream, a non-blocking one: work on another stream waits for it (an event
+ * on sph_get_stream's) or follows sph_synchronize, which also reports the
+ * updates' errors. */
 int sph_get_stream(sph_sim *sim, void **stream);
 int sph_device_arrays(sph_sim *sim, const void **pos, const void **vel, const void **dens, const void **press);
 
@@ -281,14 +284,14 @@ int sph_kernel_launches(sph_sim *sim, uint64_t *out);
  * kernel one by one instead.  Results are identical either way.  Default 1. */
 int sph_use_graphs(sph_sim *sim, int enable);
 /* No counterpart in the reference.  Launch shapes of the two ordered sweeps
- * (viscosity, delta): shape[4] = {viscosity warps per block (4 = wide,
- * 5 = lean), viscosity blocks, delta warps per block (12 = wide, 8 = mid,
- * 4 = quad, 3 = tri, 2 = lean, 16 = dense), delta blocks}.  The wide shapes
- * shorten one scene's critical path: one task per block; the wide viscosity
- * sweep runs each particle's head beside the previous particle's tail on two
- * lanes; the wide, mid, quad, tri and dense delta sweeps overlap each
- * particle's ordered sum with the next particle's pairs (11, 7, 3, 2 and 15
- * producer warps beside one summer warp; mid, quad and tri run several
+ * (viscosity, delta): shape[4] = {viscosity shape (4 = wide, 5 = lean),
+ * viscosity blocks, delta shape (12 = wide, 8 = mid, 4 = quad, 3 = tri,
+ * 2 = lean, 16 = dense), delta blocks}; the numbers name the shapes.  The wide
+ * shapes shorten one scene's critical path: one task per block; the wide
+ * viscosity sweep runs each particle's head beside the previous particle's
+ * tail on two chains; the wide, mid, quad, tri and dense delta sweeps overlap
+ * each particle's ordered sum with the next particle's pairs (12, 6, 3, 2 and
+ * 12 producer warps beside one summer warp; mid, quad and tri run several
  * blocks per SM; dense stages 12,288 entries per task, for crowded
  * states).  The lean ones
  * fit more tasks on an SM (the lean viscosity sweep runs eighteen tasks
@@ -296,7 +299,11 @@ int sph_use_graphs(sph_sim *sim, int enable);
  * shape.  sph_autotune times the
  * next update (step dt) from the current state for every shape and resident
  * block count per SM, keeps the fastest for each sweep, restores the state
- * and reports the choice; it needs a state after an update. */
+ * and reports the choice; it needs a state after an update.  The state is the
+ * particles and cells: the spring tables of a simulation with springs keep
+ * what the timed updates did to them, so a tuned run of springs differs from
+ * an untuned one (dump them before and load them after to continue as
+ * without). */
 int sph_autotune(sph_sim *sim, float dt, int *shape);
 /* Particle order of the update (single-scene simulations).  By default the
  * library renumbers particles cell by cell after every update (colour-major

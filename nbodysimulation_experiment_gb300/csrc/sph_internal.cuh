@@ -14,23 +14,18 @@ constexpr int kWarp = 32;
 // neighbour list covers.  At least kSPHMaxParticleNeighborCount (1000,
 // sph.h:69), so every scene the reference accepts fits.
 constexpr int kStageCap = 1024;
-// Particles staged per delta-sweep task: the new cells of the task's bounding
-// box grown by one (5x5 cells when particles left the cell in every
-// direction).
+// Particles staged per delta-sweep task in the wide and mid shapes: the new
+// cells of the task's bounding box grown by one (5x5 cells when particles left
+// the cell in every direction).
 constexpr int kDeltaStageCap = 4096;
 // The dense delta shape's stage: a 5x5 region of cells of ~490 particles.
 constexpr int kDeltaDenseStageCap = 12288;
-// In-range pairs buffered between the parallel geometry phase and the serial
-// chain of one particle; longer lists are drained in several rounds.
-constexpr int kChainCap = 256;
-// Per-particle inputs of the delta sweep prefetched per chunk of a task.
-constexpr int kPrefetch = 128;
 // Working array of one cell during the grid update (kSPHMaxCellParticleCount
 // is 500, sph.h:68).
 constexpr int kCellCap = 512;
 // Cells of a delta-sweep staging region (bounding box of a task's new cells,
-// grown by one) in the smaller shapes (the 8- and 16-warp shapes take 256
-// and 400).  Larger regions fall back to per-particle staging.
+// grown by one) in the wide and the smaller shapes (mid and dense take 256 and
+// 400).  Tasks with larger regions run in groups of particles whose regions fit.
 constexpr int kRegionCells = 100;
 constexpr int kMaxBodies = 100;  // kSPHMaxBodyCount, sph.h:71
 constexpr int kMaxPoly = 8;      // kMaxScenarioPolygonCount, sph.h:161

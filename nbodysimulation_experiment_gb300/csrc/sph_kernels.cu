@@ -430,8 +430,9 @@ __device__ __forceinline__ void visc_phase_bar(int threads) {
 // head to the tail.  A particle with more in-range pairs than the geometry
 // buffer holds runs its whole chain in the middle.  Its own pair, which never
 // changes a velocity (no direction), is not in the list.  One task of 36
-// particles alone: 2,101 ns per particle, 2,275 with two lanes of the block's
-// common loop, the self pair in the middle and no group on its own (visc_chain).
+// particles alone, 112 in-range pairs each and 65 on the longer chain: 1,934 ns,
+// 4,004 cycles, per particle; 8% more with two lanes of the block's common loop,
+// the self pair in the middle and no group on its own (visc_chain).
 template <class C>
 __device__ __forceinline__ void visc_chains(ViscSmemT<C> &S, int cnt, int own, int L, const StepParams &s) {
 	const int c = threadIdx.x & 1;
@@ -2083,8 +2084,8 @@ __device__ __noinline__ float2 delta_half_any(float2 xj, float2 xk, float2 pk, c
 
 // dx -= delta * 0.5 over the n buffered halves of one component, in list
 // order (demo4.cpp:251), starting at dx: one dependent subtraction per pair
-// (four cycles), in batches of 32 loaded at once, so that a batch's loads and
-// its loop branch cost little beside them.  The buffer is padded with +0 for
+// (four cycles), in batches of 32 loaded at once, so that the loads' latency and
+// the loop branch, exposed between batches, add a half and no more.  The buffer is padded with +0 for
 // kSumPad entries past n, and dx - (+0) == dx exactly.  Two lanes take a
 // component each.  In isolation 112 pairs take 685 cycles, 818 in batches of
 // eight; one lane subtracting both components took 9.4 cycles a pair.
@@ -2286,9 +2287,9 @@ __device__ __forceinline__ void produce(DeltaSmemT<C> &S, int b, int4 sl, int4 l
 // and evaluates it without compacting first, so the square root and the
 // division run beside the counting and only the halves' places wait for the
 // other warps' counts.  R is a compile-time number: a uniform branch per round
-// costs as much as the round's arithmetic.  With the two-lane sum below, one
-// task of 36 particles with 324 list entries (wide shape, alone): 1,720 cycles
-// per particle, 2,060 when every warp compacted first.
+// costs as much as the round's arithmetic.  One task of 36 particles with 324
+// list entries (wide shape, alone) takes a fifth longer per particle when every
+// warp compacts first.
 template <class C, int R>
 __device__ __forceinline__ void produce_direct(DeltaSmemT<C> &S, int b, const int *at, int own, float2 pk, int prev,
                                                uint4 below, const StepParams &s, int warp, int lane) {
@@ -2398,10 +2399,10 @@ __device__ __forceinline__ void summer(DeltaSmemT<C> &S, int b, int c, int prev,
 // Role of a warp in the pipeline: a producer's number, kProd for the summer,
 // or -1 (kApart: the summer is warp 3 and the other warps of its scheduler
 // stay out, so that no producer takes its issue slots).  The summer's dependent
-// subtractions lose a cycle whenever another warp issues in their place:
-// one task of 36 particles alone, wide shape, 799 ns per particle with three
-// warps on each scheduler and both roles in one loop, 636 apart in loops of
-// their own (dense 857 -> 637, quad 1,216 -> 1,148).
+// subtractions lose a cycle whenever another warp issues in their place: one
+// task of 36 particles alone, 112 in-range pairs each, takes 569 ns, 1,178
+// cycles, per particle in the wide shape; with three warps on each scheduler and
+// both roles in one loop a quarter more (dense a third, quad 6%).
 template <class C>
 __device__ __forceinline__ int pipeline_role(int warp) {
 	if (!C::kApart) return warp;

@@ -75,14 +75,14 @@ struct DeltaQuad {
 // Dense: pipelined, twelve producers, one block per SM, a 12,288-entry stage,
 // for crowded states where a task's region (the bounding box of its
 // particles' new cells, grown by one) outgrows the other shapes' stages and
-// their tasks would read unstaged from global memory.
+// their tasks would be staged again for every group of particles that fits.
 struct DeltaDense {
 	static constexpr int kName = 16;
 	static constexpr int kWarps = 16, kProducers = 12, kStage = kDeltaDenseStageCap, kChainW = 96, kPrefetch = 128, kMinBlocks = 1;
 	static constexpr int kRegion = 400;
 	static constexpr bool kPipelined = true, kDirect = true, kApart = true;
 };
-// Delta shapes by index (sph_set_sweep_shape names them by warp count).
+// Delta shapes by index (sph_set_sweep_shape names them by kName).
 constexpr int kDeltaShapes = 6;
 constexpr int kDeltaWide = 0, kDeltaLean = 1, kDeltaMid = 2, kDeltaTri = 3, kDeltaQuad = 4, kDeltaDense = 5;
 constexpr int delta_shape_warps(int shape) {

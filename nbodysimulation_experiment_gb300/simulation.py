@@ -126,7 +126,7 @@ class SpringParams(ctypes.Structure):
 
 SPRING_SLOTS = 16
 #: The numbers that name the ordered sweeps' launch shapes, (wide, lean) and
-#: for the delta sweep (wide, lean, mid, tri, quad, dense; its warps per task):
+#: for the delta sweep (wide, lean, mid, tri, quad, dense):
 #: the values ``sph_set_sweep_shape`` accepts (csrc/sph_kernels.cuh).
 VISC_WARPS = (4, 5)
 DELTA_WARPS = (12, 2, 8, 3, 4, 16)
